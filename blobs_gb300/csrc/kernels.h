@@ -37,6 +37,29 @@ void launch_gather_single(const WorldDev& w, const float4* A, const float4* B, c
 void launch_write_single(const WorldDev& w, float4* A, float4* B, float2* V, const float2* pos,
                          const float2* pos_old, const float2* vel, const float2* snap, cudaStream_t st);
 
+// a range of collision events put into the reference's order (events.cu)
+struct EventSort {
+  const uint4* rec;        // (substep sequence, a, b, 0), ascending substep
+  const float4* vel;
+  uint32_t n;              // events of the range
+  uint32_t seq0, n_seq;    // its substeps [seq0, seq0 + n_seq), modulo 2^32
+  uint32_t n_cols;
+  uint32_t n_buckets;      // n_seq * n_cols
+  uint32_t* count;         // n_buckets
+  uint32_t* start;         // n_buckets + 1
+  uint32_t* rank;          // n
+  uint2* member;           // n
+  uint32_t* out_a;         // n each
+  uint32_t* out_b;
+  float2* out_va;
+  float2* out_vb;
+  uint32_t* status;
+};
+void launch_ev_sort(const EventSort& s, uint32_t* tile_sums, cudaStream_t st);
+// off[k] = index of the first event of substep seq0 + min(k * stride, n_seq)
+void launch_ev_bounds(const uint4* rec, uint32_t n, uint32_t seq0, uint32_t n_seq, uint32_t stride, uint32_t* off,
+                      uint32_t n_off, cudaStream_t st);
+
 // adjoint of the single-sphere substep (adjoint.cu)
 struct AdjointSubstep {
   // recorded state at the start of the substep (t) and after it (t + 1), arena order

@@ -192,6 +192,23 @@ struct blobs_world {
   uint32_t* ev_count = nullptr;
   uint32_t* ev_seq = nullptr;
   std::deque<HostEvent> ev_host;       // drained from the device, in the reference's order
+  uint32_t ev_seq_base = 0;            // sequence number at the last drain: the buffer's events are not older
+  // events taken from the buffer and put in order on the device, not yet
+  // handed out (after those in ev_host): [off, n) of four arrays in mem,
+  // whose scratch the next batch uses again
+  struct EventBatch {
+    char* mem = nullptr;
+    size_t bytes = 0;
+    uint32_t n = 0, off = 0;
+    uint32_t *a = nullptr, *b = nullptr;
+    float2 *va = nullptr, *vb = nullptr;
+    uint32_t left() const { return n - off; }
+  } ev_batch;
+  void drop_events() {
+    ev_host.clear();
+    ev_batch.n = ev_batch.off = 0;
+    ev_seq_base = 0;
+  }
   // sorted storage keeps calculated_velocity in V, double-buffered with the
   // state, when something reads it during a step (springs, events)
   bool v_tracks() const { return has_springs || events_on; }
@@ -239,8 +256,10 @@ struct blobs_world {
     drop_snapshot();
     if (ev_mem) cudaFree(ev_mem);
     ev_mem = nullptr;
+    if (ev_batch.mem) cudaFree(ev_batch.mem);
+    ev_batch = EventBatch();
     events_on = false;
-    ev_host.clear();
+    drop_events();
     if (arena) cudaFree(arena);
     arena = nullptr;
     if (hcounters) cudaFreeHost(hcounters);
@@ -1091,6 +1110,145 @@ int read_status(blobs_world* w) {
   return BLOBS_OK;
 }
 
+// ---------------------------------------------------------------------------
+// collision events: taking the buffer's events out in the reference's order
+// ---------------------------------------------------------------------------
+constexpr uint32_t EV_BUCKETS = 1u << 22;  // buckets of one device sort: 32 MB of scratch
+
+// Which side sorts a batch: the device's fixed cost is ~25 us of launches
+// per range of EV_BUCKETS (substep, collider) buckets, the host's ~60 ns an
+// event (75k events: 4.8 ms more than the device's).  Few events, or events spread thinly over very
+// many substeps, stay with the host.
+bool sort_on_device(uint32_t n, uint32_t n_seq, uint32_t n_cols) {
+  const uint64_t per_range = std::max<uint64_t>(1, EV_BUCKETS / std::max(1u, n_cols));
+  const uint64_t ranges = (n_seq + per_range - 1) / per_range;
+  return n_seq && (uint64_t)n_cols < (1ull << 31) && n >= 512ull * ranges;
+}
+
+// The first m events left in the batch into host arrays (the velocities may
+// be NULL), ordered on the world's stream.
+cudaError_t copy_batch(blobs_world* w, uint32_t m, uint32_t* a, uint32_t* b, float* va, float* vb) {
+  const auto& x = w->ev_batch;
+  cudaStream_t st = w->st();
+  cudaError_t e = cudaMemcpyAsync(a, x.a + x.off, sizeof(uint32_t) * m, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b, x.b + x.off, sizeof(uint32_t) * m, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && va) e = cudaMemcpyAsync(va, x.va + x.off, sizeof(float2) * m, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && vb) e = cudaMemcpyAsync(vb, x.vb + x.off, sizeof(float2) * m, cudaMemcpyDeviceToHost, st);
+  return e;
+}
+
+// What is left of the batch to the end of ev_host.
+cudaError_t spill_batch(blobs_world* w) {
+  auto& x = w->ev_batch;
+  const uint32_t m = x.left();
+  if (!m) return cudaSuccess;
+  std::vector<uint32_t> a(m), b(m);
+  std::vector<float2> va(m), vb(m);
+  cudaError_t e = copy_batch(w, m, a.data(), b.data(), &va[0].x, &vb[0].x);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(w->st());
+  if (e != cudaSuccess) return e;
+  for (uint32_t k = 0; k < m; ++k)
+    w->ev_host.push_back({a[k], b[k], {va[k].x, va[k].y}, {vb[k].x, vb[k].y}});
+  x.n = x.off = 0;
+  return cudaSuccess;
+}
+
+// All n events of the buffer to the end of ev_host, sorted on the host.
+cudaError_t take_events_host(blobs_world* w, uint32_t n) {
+  cudaStream_t st = w->st();
+  std::vector<uint4> rec(n);
+  std::vector<float4> vel(n);
+  cudaError_t e = cudaMemcpyAsync(rec.data(), w->ev_rec, sizeof(uint4) * n, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(vel.data(), w->ev_vel, sizeof(float4) * n, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
+  std::vector<uint32_t> order(n);
+  std::iota(order.begin(), order.end(), 0u);
+  std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+    const uint4 &p = rec[x], &q = rec[y];
+    if (p.x != q.x) return (int32_t)(p.x - q.x) < 0;  // sequence, modulo 2^32
+    if (p.y != q.y) return p.y < q.y;
+    return p.z < q.z;
+  });
+  for (uint32_t k : order)
+    w->ev_host.push_back({rec[k].y, rec[k].z, {vel[k].x, vel[k].y}, {vel[k].z, vel[k].w}});
+  return cudaSuccess;
+}
+
+// All n events of the buffer (substeps ev_seq_base .. + n_seq) into the
+// batch, sorted by the device (events.cu) in ranges of whole substeps.
+cudaError_t take_events_device(blobs_world* w, uint32_t n, uint32_t n_seq) {
+  cudaStream_t st = w->st();
+  auto& x = w->ev_batch;
+  const uint32_t nc = w->nc;
+  const uint32_t per = std::min(n_seq, std::max(1u, EV_BUCKETS / nc));  // substeps of a range
+  const uint32_t ranges = (n_seq + per - 1) / per, nb = per * nc;
+  EventSort s{};
+  uint32_t *tiles = nullptr, *off = nullptr;
+  auto lay = [&](Carver& c) {
+    x.a = c.take<uint32_t>(n);
+    x.b = c.take<uint32_t>(n);
+    x.va = c.take<float2>(n);
+    x.vb = c.take<float2>(n);
+    s.rank = c.take<uint32_t>(n);
+    s.member = c.take<uint2>(n);
+    s.count = c.take<uint32_t>(nb);
+    s.start = c.take<uint32_t>((size_t)nb + 1);
+    tiles = c.take<uint32_t>((nb + SCAN_TILE - 1) / SCAN_TILE);
+    off = c.take<uint32_t>((size_t)ranges + 1);
+  };
+  Carver sizer;
+  lay(sizer);
+  if (x.bytes < sizer.off) {
+    // grown by half, so that a slowly growing stream does not reallocate on each drain
+    const size_t want = sizer.off + sizer.off / 2 + 256;
+    if (x.mem) cudaFree(x.mem);
+    x = blobs_world::EventBatch();
+    cudaError_t e = cudaMalloc(&x.mem, want);
+    if (e != cudaSuccess) {
+      x.mem = nullptr;
+      return e;
+    }
+    x.bytes = want;
+  }
+  Carver cv;
+  cv.base = x.mem;
+  lay(cv);
+  std::vector<uint32_t> first(ranges + 1, 0);
+  first[ranges] = n;
+  if (ranges > 1) {
+    launch_ev_bounds(w->ev_rec, n, w->ev_seq_base, n_seq, per, off, ranges + 1, st);
+    cudaError_t e = cudaMemcpyAsync(first.data(), off, sizeof(uint32_t) * (ranges + 1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    for (uint32_t r = 0; r < ranges; ++r)
+      if (first[r] > first[r + 1] || first[r + 1] > n) return cudaErrorUnknown;
+  }
+  uint32_t* rank = s.rank;
+  uint2* member = s.member;
+  for (uint32_t r = 0; r < ranges; ++r) {
+    const uint32_t e0 = first[r];
+    s.rec = w->ev_rec + e0;
+    s.vel = w->ev_vel + e0;
+    s.n = first[r + 1] - e0;
+    s.seq0 = w->ev_seq_base + r * per;
+    s.n_seq = std::min(per, n_seq - r * per);
+    s.n_cols = nc;
+    s.n_buckets = s.n_seq * nc;
+    s.rank = rank + e0;
+    s.member = member + e0;
+    s.out_a = x.a + e0;
+    s.out_b = x.b + e0;
+    s.out_va = x.va + e0;
+    s.out_vb = x.vb + e0;
+    s.status = w->dev.status;
+    launch_ev_sort(s, tiles, st);
+  }
+  x.n = n;
+  x.off = 0;
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1332,7 +1490,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   w->attach_events();
   if (w->events_on) {
     // a reloaded world starts a new event stream
-    w->ev_host.clear();
+    w->drop_events();
     cudaMemsetAsync(w->ev_count, 0, 2 * sizeof(uint32_t), s);
   }
   w->nb = nb;
@@ -1878,7 +2036,9 @@ int blobs_world_set_events(blobs_world* w, int enabled, uint32_t capacity) {
   w->drop_recording();  // checkpoints hold V in the previous mode
   if (w->ev_mem) cudaFree(w->ev_mem);
   w->ev_mem = nullptr;
-  w->ev_host.clear();
+  if (w->ev_batch.mem) cudaFree(w->ev_batch.mem);
+  w->ev_batch = blobs_world::EventBatch();
+  w->drop_events();
   w->events_on = false;
   if (enabled) {
     Carver sizer;
@@ -1933,43 +2093,33 @@ int blobs_world_drain_events(blobs_world* w, uint32_t* col_a, uint32_t* col_b, f
   e = cudaMemcpyAsync(head, w->ev_count, sizeof(head), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return blobs_map_cuda(e);
-  const uint32_t n = head[0];
+  const uint32_t n = head[0], n_seq = head[1] - w->ev_seq_base;
   if (n > w->ev_cap) {
     // the appended subset is not a prefix of the reference order: drop it
     e = cudaMemsetAsync(w->ev_count, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    w->ev_seq_base = head[1];
     if (n_left) *n_left = n;
     return e == cudaSuccess ? BLOBS_ERR_OVERFLOW : blobs_map_cuda(e);
   }
   if (n) {
-    std::vector<uint4> rec(n);
-    std::vector<float4> vel(n);
-    e = cudaMemcpyAsync(rec.data(), w->ev_rec, sizeof(uint4) * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(vel.data(), w->ev_vel, sizeof(float4) * n, cudaMemcpyDeviceToHost, st);
+    e = spill_batch(w);  // an earlier batch comes first
+    if (e == cudaSuccess) {
+      bool on_host = !sort_on_device(n, n_seq, w->nc);
+      if (!on_host) {
+        e = take_events_device(w, n, n_seq);
+        if (e == cudaErrorMemoryAllocation) {  // no room for the scratch
+          cudaGetLastError();
+          on_host = true;
+        }
+      }
+      if (on_host) e = take_events_host(w, n);
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(w->ev_count, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return blobs_map_cuda(e);
-    // the reference's order: substep by substep, outer collider ascending,
-    // inner collider ascending (physics.rs:247-248)
-    std::vector<uint32_t> order(n);
-    std::iota(order.begin(), order.end(), 0u);
-    std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-      const uint4 &p = rec[x], &q = rec[y];
-      if (p.x != q.x) return (int32_t)(p.x - q.x) < 0;  // sequence, modulo 2^32
-      if (p.y != q.y) return p.y < q.y;
-      return p.z < q.z;
-    });
-    for (uint32_t k : order) {
-      blobs_world::HostEvent ev;
-      ev.a = rec[k].y;
-      ev.b = rec[k].z;
-      ev.va[0] = vel[k].x;
-      ev.va[1] = vel[k].y;
-      ev.vb[0] = vel[k].z;
-      ev.vb[1] = vel[k].w;
-      w->ev_host.push_back(ev);
-    }
   }
+  w->ev_seq_base = head[1];
   uint64_t k = 0;
   while (k < cap && !w->ev_host.empty()) {
     const blobs_world::HostEvent& ev = w->ev_host.front();
@@ -1980,8 +2130,17 @@ int blobs_world_drain_events(blobs_world* w, uint32_t* col_a, uint32_t* col_b, f
     w->ev_host.pop_front();
     ++k;
   }
+  auto& b = w->ev_batch;
+  const uint32_t m = (uint32_t)std::min<uint64_t>(cap - k, b.left());
+  if (m) {
+    e = copy_batch(w, m, col_a + k, col_b + k, impact_vel_a ? impact_vel_a + 2 * k : nullptr,
+                   impact_vel_b ? impact_vel_b + 2 * k : nullptr);
+    if (e != cudaSuccess) return blobs_map_cuda(e);
+    b.off += m;
+    k += m;
+  }
   *n_written = k;
-  if (n_left) *n_left = w->ev_host.size();
+  if (n_left) *n_left = w->ev_host.size() + b.left();
   return read_status(w);
 }
 
