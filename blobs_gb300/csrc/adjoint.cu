@@ -31,6 +31,7 @@
 namespace blobs {
 
 __global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) {
+  pdl_enter();
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= w.n_bodies) return;
   const uint8_t fl = w.bflags[b];
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) 
 }
 
 __global__ void __launch_bounds__(256) k_adj_springs(WorldDev w, AdjointSubstep a) {
+  pdl_enter();
   const uint32_t sidx = blockIdx.x * blockDim.x + threadIdx.x;
   if (sidx >= w.n_springs) return;
   a.spr_terms[sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(256) k_adj_springs(WorldDev w, AdjointSubstep 
 }
 
 __global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a) {
+  pdl_enter();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= w.n_bodies) return;
   // contacts: p_c(hi) += rho d(n) ... on s_hi - s_lo, evaluated from this body's side
@@ -176,9 +179,9 @@ __global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a
 
 void launch_adjoint_substep(const WorldDev& w, const AdjointSubstep& a, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_adj_body<<<(w.n_bodies + 255u) / 256u, 256, 0, st>>>(w, a);
-  if (w.n_springs) k_adj_springs<<<(w.n_springs + 255u) / 256u, 256, 0, st>>>(w, a);
-  k_adj_gather<<<(w.n_bodies + 255u) / 256u, 256, 0, st>>>(w, a);
+  launch_pdl(k_adj_body, (w.n_bodies + 255u) / 256u, 256, st, true, w, a);
+  if (w.n_springs) launch_pdl(k_adj_springs, (w.n_springs + 255u) / 256u, 256, st, true, w, a);
+  launch_pdl(k_adj_gather, (w.n_bodies + 255u) / 256u, 256, st, true, w, a);
 }
 
 }  // namespace blobs

@@ -152,6 +152,20 @@ struct WorldDev {
   uint32_t* status;
 };
 
+// First statement, before any read of memory, of the kernels that launch_pdl
+// (kernels.h) starts: waits until the kernels before it are complete and
+// their writes visible, then lets the next kernel in the stream be placed on
+// the SMs once all blocks of this one have come this far.  A single-sphere
+// substep is five dependent kernels, a few microseconds each in small
+// worlds; the launch of one hides behind the run of the one before it (1M
+// sparse spheres: 2.28 -> 2.19 ms for four steps; the eager launches of a
+// small gradient: 1.76 -> 1.33 ms).  The trigger stands after the wait:
+// before it, whole chains of waiting kernels filled the SMs.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // glam Vec2 arithmetic, one rounding per operation.
 // ---------------------------------------------------------------------------

@@ -29,6 +29,7 @@ __device__ __forceinline__ uint32_t event_bucket(const EventSort& s, uint4 r) {
 __global__ void __launch_bounds__(256) k_ev_bounds(const uint4* __restrict__ rec, uint32_t n, uint32_t seq0,
                                                    uint32_t n_seq, uint32_t stride, uint32_t* __restrict__ off,
                                                    uint32_t n_off) {
+  pdl_enter();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_off) return;
   const uint32_t want = min(k * stride, n_seq);
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(256) k_ev_bounds(const uint4* __restrict__ rec
 }
 
 __global__ void __launch_bounds__(256) k_ev_count(EventSort s) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
   const uint32_t k = event_bucket(s, s.rec[i]);
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(256) k_ev_count(EventSort s) {
 
 // member[slot] = (b, event) of the event at its place among the buckets
 __global__ void __launch_bounds__(256) k_ev_place(EventSort s) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
   const uint4 r = s.rec[i];
@@ -63,6 +66,7 @@ __global__ void __launch_bounds__(256) k_ev_place(EventSort s) {
 // one thread per event: its rank by b inside its bucket is its place
 // (pairs are distinct; the slot breaks ties so that ranks stay a permutation)
 __global__ void __launch_bounds__(256) k_ev_write(EventSort s) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
   const uint4 r = s.rec[i];
@@ -84,23 +88,23 @@ __global__ void __launch_bounds__(256) k_ev_write(EventSort s) {
 
 void launch_ev_bounds(const uint4* rec, uint32_t n, uint32_t seq0, uint32_t n_seq, uint32_t stride, uint32_t* off,
                       uint32_t n_off, cudaStream_t st) {
-  k_ev_bounds<<<(n_off + 255u) / 256u, 256, 0, st>>>(rec, n, seq0, n_seq, stride, off, n_off);
+  launch_pdl(k_ev_bounds, (n_off + 255u) / 256u, 256, st, true, rec, n, seq0, n_seq, stride, off, n_off);
 }
 
 void launch_ev_sort(const EventSort& s, uint32_t* tile_sums, cudaStream_t st) {
   if (!s.n) return;
   const uint32_t g = (s.n + 255u) / 256u;
   cudaMemsetAsync(s.count, 0, sizeof(uint32_t) * (size_t)s.n_buckets, st);
-  k_ev_count<<<g, 256, 0, st>>>(s);
+  launch_pdl(k_ev_count, g, 256, st, true, s);
   WorldDev d{};  // the cell scan over the buckets
   d.cell_count = s.count;
   d.cell_start = s.start;
   d.n_cells = s.n_buckets;
   d.n_tiles = (s.n_buckets + SCAN_TILE - 1) / SCAN_TILE;
   d.tile_sums = tile_sums;
-  launch_scan(d, st);
-  k_ev_place<<<g, 256, 0, st>>>(s);
-  k_ev_write<<<g, 256, 0, st>>>(s);
+  launch_scan(d, st, true);
+  launch_pdl(k_ev_place, g, 256, st, true, s);
+  launch_pdl(k_ev_write, g, 256, st, true, s);
 }
 
 }  // namespace blobs

@@ -86,6 +86,7 @@ __device__ __forceinline__ void load_tile(const WorldDev& w, size_t base, uint32
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(WorldDev w) {
+  pdl_enter();
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
   uint32_t v[SCAN_ITEMS];
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(WorldDev w) {
 // their exclusive prefix in place, so that k_scan_apply reads its prefix
 // instead of summing all earlier tiles (quadratic in the tile count).
 __global__ void __launch_bounds__(1024) k_tile_prefix(WorldDev w) {
+  pdl_enter();
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_carry;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(1024) k_tile_prefix(WorldDev w) {
 
 template <bool PREFIXED>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(WorldDev w) {
+  pdl_enter();
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ uint32_t s_prefix;
   if (PREFIXED) {
@@ -758,19 +761,21 @@ __global__ void __launch_bounds__(256) k_body_contacts(WorldDev w, const float2*
 
 // Advances the collision-event substep sequence (after a contact pass).
 __global__ void k_ev_tick(WorldDev w) {
+  pdl_enter();
   if (threadIdx.x == 0) *w.ev_seq += 1u;
 }
 
-void launch_ev_tick(const WorldDev& w, cudaStream_t st) { k_ev_tick<<<1, 32, 0, st>>>(w); }
+void launch_ev_tick(const WorldDev& w, cudaStream_t st) { launch_pdl(k_ev_tick, 1, 32, st, true, w); }
 
 // Divides a V buffer of displacements by dt in place (storage order).
 __global__ void k_v_divide(float2* v, uint32_t n, float dt) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) v[i] = divs(v[i], dt);
 }
 
 void launch_v_divide(float2* v, uint32_t n, float dt, cudaStream_t st) {
-  if (n) k_v_divide<<<(n + 255u) / 256u, 256, 0, st>>>(v, n, dt);
+  if (n) launch_pdl(k_v_divide, (n + 255u) / 256u, 256, st, true, v, n, dt);
 }
 
 // ---------------------------------------------------------------------------
@@ -1025,15 +1030,15 @@ void launch_keys(const WorldDev& w, bool mw, cudaStream_t st) {
   else k_keys<false><<<g, 256, 0, st>>>(w);
 }
 
-uint32_t launch_scan(const WorldDev& w, cudaStream_t st) {
+uint32_t launch_scan(const WorldDev& w, cudaStream_t st, bool early) {
   const uint32_t tiles = blocks_for(w.n_cells, SCAN_TILE);
-  k_tile_sums<<<tiles, SCAN_THREADS, 0, st>>>(w);
+  launch_pdl(k_tile_sums, tiles, SCAN_THREADS, st, early, w);
   if (tiles > SCAN_PREFIX_TILES && tiles == w.n_tiles) {
-    k_tile_prefix<<<1, 1024, 0, st>>>(w);
-    k_scan_apply<true><<<tiles, SCAN_THREADS, 0, st>>>(w);
+    launch_pdl(k_tile_prefix, 1, 1024, st, early, w);
+    launch_pdl(k_scan_apply<true>, tiles, SCAN_THREADS, st, early, w);
     return 3;
   }
-  k_scan_apply<false><<<tiles, SCAN_THREADS, 0, st>>>(w);
+  launch_pdl(k_scan_apply<false>, tiles, SCAN_THREADS, st, early, w);
   return 2;
 }
 

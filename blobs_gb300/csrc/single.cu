@@ -538,6 +538,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
 
 // Storage slot i -> its position in this substep's cell order.
 __global__ void __launch_bounds__(256) k_permute(WorldDev w, SingleArgs a) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= w.n_bodies) return;
   const uint32_t key = w.key[i];
@@ -558,6 +559,7 @@ __global__ void __launch_bounds__(256) k_permute(WorldDev w, SingleArgs a) {
 // Cell-order copy of the snapshot records (candidates of this substep).
 __global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* __restrict__ a_in,
                                                       float4* __restrict__ cand) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= w.n_bodies) return;
   const uint32_t j = w.cell_start[w.key[i]] + w.rank[i];
@@ -576,6 +578,7 @@ __global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* 
 // O(contacts x candidates) walk or the O(near^2) ordered selection.
 template <int MODE, bool HOOKS>
 __global__ void __launch_bounds__(STEP_THREADS, 8) k_step_single(WorldDev w, SingleArgs a) {
+  pdl_enter();
   // phase 2 shared out over the warp (apply_near_warp): the plain step of a
   // uniform world
   constexpr bool WARP2 = MODE == 0 && !HOOKS;
@@ -803,6 +806,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 8) k_step_single(WorldDev w, Sin
 // the exact selection walk on one lane.
 template <int MODE, bool HOOKS>
 __global__ void __launch_bounds__(DEFER_THREADS) k_step_deferred(WorldDev w, SingleArgs a) {
+  pdl_enter();
   __shared__ DeferWarp dsm[DEFER_THREADS / 32];
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   DeferWarp& S = dsm[wib];
@@ -936,6 +940,7 @@ __global__ void __launch_bounds__(DEFER_THREADS) k_step_deferred(WorldDev w, Sin
 
 // Keys and ranks of the current storage (after a load or a host write).
 __global__ void __launch_bounds__(256) k_keys_single(WorldDev w, const float4* __restrict__ A, int mode) {
+  pdl_enter();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= w.n_bodies) return;
   const float4 a = A[j];
@@ -951,6 +956,7 @@ __global__ void __launch_bounds__(256) k_gather_single(WorldDev w, const float4*
                                                        const float4* __restrict__ B, const float2* __restrict__ V,
                                                        float2* pos, float2* pos_old, float2* vel, float2* snap,
                                                        float v_div) {
+  pdl_enter();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= w.n_bodies) return;
   const float4 a = A[j];
@@ -974,6 +980,7 @@ __global__ void __launch_bounds__(256) k_gather_single(WorldDev w, const float4*
 __global__ void __launch_bounds__(256) k_write_single(WorldDev w, float4* A, float4* B, float2* V,
                                                       const float2* pos, const float2* pos_old, const float2* vel,
                                                       const float2* snap) {
+  pdl_enter();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= w.n_bodies) return;
   const uint32_t c = __float_as_uint(A[j].w);
@@ -1006,56 +1013,59 @@ static inline uint32_t nblocks(uint32_t n) { return (n + 255u) / 256u; }
 
 void launch_permute(const WorldDev& w, const SingleArgs& a, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_permute<<<nblocks(w.n_bodies), 256, 0, st>>>(w, a);
+  launch_pdl(k_permute, nblocks(w.n_bodies), 256, st, true, w, a);
 }
 
 void launch_scatter_cand(const WorldDev& w, const float4* a_in, float4* cand, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_scatter_cand<<<nblocks(w.n_bodies), 256, 0, st>>>(w, a_in, cand);
+  launch_pdl(k_scatter_cand, nblocks(w.n_bodies), 256, st, true, w, a_in, cand);
 }
 
 void launch_step_single(const WorldDev& w, const SingleArgs& a, int mode, cudaStream_t st) {
   if (!w.n_bodies) return;
   const uint32_t g = (w.n_bodies + STEP_THREADS - 1) / STEP_THREADS;
   if (a.rec_list || w.ev_rec) {
-    if (mode == 0) k_step_single<0, true><<<g, STEP_THREADS, 0, st>>>(w, a);
-    else if (mode == 1) k_step_single<1, true><<<g, STEP_THREADS, 0, st>>>(w, a);
-    else k_step_single<2, true><<<g, STEP_THREADS, 0, st>>>(w, a);
+    if (mode == 0) launch_pdl(k_step_single<0, true>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_single<1, true>, g, STEP_THREADS, st, true, w, a);
+    else launch_pdl(k_step_single<2, true>, g, STEP_THREADS, st, true, w, a);
   } else {
-    if (mode == 0) k_step_single<0, false><<<g, STEP_THREADS, 0, st>>>(w, a);
-    else if (mode == 1) k_step_single<1, false><<<g, STEP_THREADS, 0, st>>>(w, a);
-    else k_step_single<2, false><<<g, STEP_THREADS, 0, st>>>(w, a);
+    if (mode == 0) launch_pdl(k_step_single<0, false>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_single<1, false>, g, STEP_THREADS, st, true, w, a);
+    else launch_pdl(k_step_single<2, false>, g, STEP_THREADS, st, true, w, a);
   }
 }
 
 void launch_step_deferred(const WorldDev& w, const SingleArgs& a, int mode, cudaStream_t st) {
   if (!w.n_bodies || !w.defer_list) return;
+  // a warp for every body at most: a 1,000-sphere world's 1,216 blocks were
+  // mostly the time of starting them
+  const uint32_t g = min(DEFER_BLOCKS, (w.n_bodies + DEFER_THREADS / 32 - 1) / (DEFER_THREADS / 32));
   if (a.rec_list || w.ev_rec) {
-    if (mode == 0) k_step_deferred<0, true><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
-    else if (mode == 1) k_step_deferred<1, true><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
-    else k_step_deferred<2, true><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
+    if (mode == 0) launch_pdl(k_step_deferred<0, true>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_deferred<1, true>, g, DEFER_THREADS, st, true, w, a);
+    else launch_pdl(k_step_deferred<2, true>, g, DEFER_THREADS, st, true, w, a);
   } else {
-    if (mode == 0) k_step_deferred<0, false><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
-    else if (mode == 1) k_step_deferred<1, false><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
-    else k_step_deferred<2, false><<<DEFER_BLOCKS, DEFER_THREADS, 0, st>>>(w, a);
+    if (mode == 0) launch_pdl(k_step_deferred<0, false>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_deferred<1, false>, g, DEFER_THREADS, st, true, w, a);
+    else launch_pdl(k_step_deferred<2, false>, g, DEFER_THREADS, st, true, w, a);
   }
 }
 
 void launch_keys_single(const WorldDev& w, const float4* A, int mode, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_keys_single<<<nblocks(w.n_bodies), 256, 0, st>>>(w, A, mode);
+  launch_pdl(k_keys_single, nblocks(w.n_bodies), 256, st, true, w, A, mode);
 }
 
 void launch_gather_single(const WorldDev& w, const float4* A, const float4* B, const float2* V, float2* pos,
                           float2* pos_old, float2* vel, float2* snap, float v_div, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_gather_single<<<nblocks(w.n_bodies), 256, 0, st>>>(w, A, B, V, pos, pos_old, vel, snap, v_div);
+  launch_pdl(k_gather_single, nblocks(w.n_bodies), 256, st, true, w, A, B, V, pos, pos_old, vel, snap, v_div);
 }
 
 void launch_write_single(const WorldDev& w, float4* A, float4* B, float2* V, const float2* pos,
                          const float2* pos_old, const float2* vel, const float2* snap, cudaStream_t st) {
   if (!w.n_bodies) return;
-  k_write_single<<<nblocks(w.n_bodies), 256, 0, st>>>(w, A, B, V, pos, pos_old, vel, snap);
+  launch_pdl(k_write_single, nblocks(w.n_bodies), 256, st, true, w, A, B, V, pos, pos_old, vel, snap);
 }
 
 }  // namespace blobs

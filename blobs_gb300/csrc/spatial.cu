@@ -52,6 +52,7 @@ struct HashDev {
 };
 
 __global__ void __launch_bounds__(256) k_sh_keys(HashDev h) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= h.n) return;
   const float2 p = h.xy[i];
@@ -63,6 +64,7 @@ __global__ void __launch_bounds__(256) k_sh_keys(HashDev h) {
 }
 
 __global__ void __launch_bounds__(256) k_sh_scatter(HashDev h, uint32_t* status) {
+  pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= h.n) return;
   const uint32_t s = h.start[h.bucket[i]] + h.rank[i];
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(256) k_sh_query(HashDev h, const unsigned long
                                                   const float* __restrict__ qr, uint32_t* qcount,
                                                   const uint32_t* qstart, unsigned long long* out,
                                                   unsigned long long cap) {
+  pdl_enter();
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) return;
   const float2 x = qxy[q];
@@ -153,7 +156,7 @@ void scan_counts(uint32_t* count, uint32_t* start, uint32_t n, uint32_t* tile_su
   d.tile_sums = tile_sums;
   d.contacts_sub = sub_bins;
   d.defer_sub = sub_bins;
-  launch_scan(d, st);
+  launch_scan(d, st, true);
 }
 
 }  // namespace
@@ -305,9 +308,9 @@ int blobs_spatial_hash_set_points(blobs_spatial_hash* h, uint64_t n, const uint6
   if (e == cudaSuccess) e = cudaMemsetAsync(h->status, 0, 4, st);
   if (e != cudaSuccess) return blobs_map_cuda(e);
   const HashDev d = h->dev();
-  if (n) k_sh_keys<<<nblk(n), 256, 0, st>>>(d);
+  if (n) launch_pdl(k_sh_keys, nblk(n), 256, st, true, d);
   scan_counts(h->count, h->start, nb, h->tile_sums, h->sub_bins, st);
-  if (n) k_sh_scatter<<<nblk(n), 256, 0, st>>>(d, h->status);
+  if (n) launch_pdl(k_sh_scatter, nblk(n), 256, st, true, d, h->status);
   uint32_t status = 0;
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(&status, h->status, 4, cudaMemcpyDeviceToHost, st);
@@ -352,7 +355,7 @@ int blobs_spatial_hash_query(blobs_spatial_hash* h, uint64_t nq, const float* qx
   if (e == cudaSuccess) e = cudaMemcpyAsync(dr, qradius, 4 * nq, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return blobs_map_cuda(e);
   const HashDev d = h->dev();
-  k_sh_query<false><<<nblk(nq), 256, 0, st>>>(d, h->ids, (uint32_t)nq, dq, dr, qcount, nullptr, nullptr, 0ull);
+  launch_pdl(k_sh_query<false>, nblk(nq), 256, st, true, d, h->ids, (uint32_t)nq, dq, dr, qcount, nullptr, nullptr, 0ull);
   // totals above 2^32 - 1 would wrap the u32 scan: refused below
   scan_counts(qcount, qstart, (uint32_t)nq, tiles, bins, st);
   std::vector<uint32_t> hstart(nq + 1);
@@ -372,7 +375,7 @@ int blobs_spatial_hash_query(blobs_spatial_hash* h, uint64_t nq, const float* qx
   e = ensure(&h->omem, &h->omem_bytes, 8 * run);
   if (e != cudaSuccess) return blobs_map_cuda(e);
   unsigned long long* dout = static_cast<unsigned long long*>(h->omem);
-  k_sh_query<true><<<nblk(nq), 256, 0, st>>>(d, h->ids, (uint32_t)nq, dq, dr, nullptr, qstart, dout, run);
+  launch_pdl(k_sh_query<true>, nblk(nq), 256, st, true, d, h->ids, (uint32_t)nq, dq, dr, nullptr, qstart, dout, run);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(ids, dout, 8 * run, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -878,7 +878,7 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
         w->enqueued += 1;
       }
       mark_begin(w, PHASE_SCAN);
-      w->enqueued += launch_scan(d, st);
+      w->enqueued += launch_scan(d, st, true);
       mark_end(w);
       mark_begin(w, PHASE_SCATTER);
       if (first_in_step) {
@@ -935,7 +935,7 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
   }
   if (coll) {
     mark_begin(w, PHASE_SCAN);
-    w->enqueued += launch_scan(d, st);
+    w->enqueued += launch_scan(d, st, false);
     mark_end(w);
   }
   if (coll || w->has_springs) {
@@ -1769,7 +1769,7 @@ int blobs_world_emit_pairs(blobs_world* w, int contacts_only, uint32_t* pairs, u
   if (w->sorted_storage) {
     const int c = (int)w->cur;
     if (!w->keys_valid) launch_keys_single(w->dev, w->dev.sa[c], w->single_mode, s);
-    launch_scan(w->dev, s);
+    launch_scan(w->dev, s, true);
     SingleArgs a;
     std::memset(&a, 0, sizeof(a));
     a.a_in = w->dev.sa[c];
@@ -1787,7 +1787,7 @@ int blobs_world_emit_pairs(blobs_world* w, int contacts_only, uint32_t* pairs, u
     dv.sorted = w->dev.sa[w->cur];
   } else {
     if (!w->keys_valid) launch_keys(w->dev, w->multiworld, s);
-    launch_scan(w->dev, s);
+    launch_scan(w->dev, s, false);
     launch_scatter_forces(w->dev, w->pos[w->cur], w->multiworld, true, false, false, s);
   }
   w->keys_valid = false;
