@@ -284,9 +284,10 @@ int blobs_world_rollout_record(blobs_world* w, double delta, uint32_t n_steps, u
  * physics.rs:272-286) are not differentiated.  The world is left in the
  * rollout's final state.  A reload, a change of the substep count or of the
  * event mode drops the recording (then BLOBS_ERR_STATE).  Every sum runs
- * in a fixed order: the gradients are deterministic.  Allocates its scratch
- * per call: 92 B per body per substep of one checkpoint segment (the state
- * after the substep and up to 16 recorded contacts); a body with more than
+ * in a fixed order: the gradients are deterministic.  Its scratch is 92 B per
+ * body per substep of one checkpoint segment (the state after the substep
+ * and up to 16 recorded contacts), taken for the call from a pool that keeps
+ * up to 8 GB per device for the next one; a body with more than
  * 16 contacts in one substep gives BLOBS_ERR_OVERFLOW.  The derivative of
  * long contact-rich rollouts can exceed the f32 range; such gradients come
  * back as +-inf or NaN with BLOBS_OK.  Synchronising. */
