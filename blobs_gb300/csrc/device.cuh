@@ -36,7 +36,7 @@ struct WorldParam {
   float box_lo_x, box_lo_y, box_hi_x, box_hi_y;
   uint32_t has_box;     // axis-aligned wall extension enabled
   float inv_cs;         // 1 / cs (rounded once, on the host)
-  uint32_t first_dyn;   // arena id of the world's first non-static body (uniform single-sphere worlds)
+  uint32_t first_dyn;   // arena id of this world's first non-static body (uniform single-sphere worlds)
   float uniform_gmod;   // gravity_mod shared by every body (uniform single-sphere worlds)
   float ox, oy;         // grid origin: the world's extent maps to cells 1 .. W-2, away from the wrap
   uint32_t pad[2];
@@ -73,6 +73,9 @@ struct WorldDev {
   uint32_t* body_cols;
   uint32_t* body_spr_start;  // n_bodies + 1: incident springs, ascending spring index
   uint32_t* body_spr;        // (spring index << 1) | (1 if the body is endpoint b)
+  uint32_t n_spr_bodies;     // single-sphere path: bodies with springs,
+  uint32_t* spr_bodies;      // their arena ids, ascending,
+  uint32_t* spr_bits;        // and a bit for each body that is one of them
 
   // colliders (arena order)
   uint32_t* col_parent;
@@ -114,6 +117,9 @@ struct WorldDev {
 
   // broadphase
   uint32_t* cell_count;      // n_cells, zero between substeps
+  uint32_t* key_b;           // resident kernel: second buffers of key and rank,
+  uint32_t* rank_b;
+  uint32_t* cell_count_b;    // and two more of cell_count (2 n_cells), zero between launches
   uint32_t* cell_start;      // n_cells + 1
   uint32_t* rank;            // per collider: slot inside its cell
   float4* sorted;            // per slot: (x, y, radius, collider index bits)
@@ -286,6 +292,11 @@ struct SingleArgs {
   float2* v_out;
   const float4* cand;        // candidate records in cell order
   const uint32_t* own_cell;  // cell of each storage slot in this substep's order
+  const uint32_t* cell_start;  // the substep's cell table (indexed by global cell),
+  uint32_t* cell_count;        // the counts of the next substep,
+  uint32_t* key_out;           // the bodies' cells and ranks there,
+  uint32_t* rank_out;
+  const WorldParam* wparam;    // and the worlds' parameters
   float dt, ratio_first, ratio_rest;
   uint32_t contacts, pending, springs, rot_dynamic, do_keys, write_v, move_v;
   uint32_t v_vel;            // V holds calculated_velocity (else the displacement of the last substep)
@@ -298,6 +309,20 @@ struct SingleArgs {
   uint32_t* rec_list;
   uint32_t* rec_n;
   uint32_t* rec_max;
+};
+
+// A world of the resident kernel: its bodies are storage slots
+// [body0, body0 + n_bodies).
+struct ResWorld {
+  uint32_t world, body0, n_bodies, pad;
+};
+
+struct ResidentArgs {
+  SingleArgs base;           // constants of the steps; pending and ratio_first: of the launch's first substep
+  const ResWorld* worlds;
+  uint32_t cluster;          // blocks per world
+  uint32_t n_steps, substeps;
+  uint32_t cur, vbuf;        // storage buffer holding the state, V buffer when V is not tracked
 };
 
 // Append one collision event (physics.rs:304-311): the pair (a, b) with
@@ -328,6 +353,11 @@ constexpr uint32_t CL_CAP = 8;             // general path: contacts kept per co
 constexpr uint32_t COUNTER_BINS = 64;
 constexpr uint32_t REC_CAP = 16;           // recorded contacts per body and substep (adjoint)
 constexpr int JB_THREADS = 128;            // k_joint_blocks: one thread per small component
+constexpr uint32_t RES_THREADS = 256;      // resident kernel: threads of a block,
+constexpr uint32_t RES_PER_THREAD = 2;     // bodies of a thread at most,
+constexpr uint32_t RES_MAX_CLUSTER = 8;    // blocks of a world at most,
+constexpr uint32_t RES_MAX_BODIES = RES_THREADS * RES_PER_THREAD * RES_MAX_CLUSTER;  // bodies of a world
+constexpr uint32_t RES_MAX_CELLS = 2 * RES_MAX_BODIES;  // and cells (what the grid cap gives that many bodies)
 constexpr uint32_t JB_MAX_JOINTS = 64;     // larger components take the coloured sweep
 constexpr uint32_t JB_JOINTS = 512;        // joints staged in shared memory per block
 constexpr uint32_t JB_BODIES = 640;        // bodies staged per block (<= JB_JOINTS + JB_THREADS)

@@ -44,12 +44,18 @@ void launch_emit_pairs(const WorldDev& w, bool multiworld, uint32_t mode, uint32
                        unsigned long long* count, cudaStream_t st);
 
 // single-sphere path with cell-sorted storage (single.cu); mode 0: one
-// uniform world, 1: one world with per-body records, 2: batched worlds
+// uniform world, 1: one world with per-body records, 2: batched worlds, 3:
+// batched uniform worlds
 void launch_permute(const WorldDev& w, const SingleArgs& a, cudaStream_t st);
-void launch_scatter_cand(const WorldDev& w, const float4* a_in, float4* cand, cudaStream_t st);
+// with springs also the spring forces of the substep; launch_springs: those alone
+void launch_scatter_cand(const WorldDev& w, const SingleArgs& a, float4* cand, cudaStream_t st);
+void launch_springs(const WorldDev& w, const SingleArgs& a, cudaStream_t st);
 void launch_step_single(const WorldDev& w, const SingleArgs& a, int mode, cudaStream_t st);
 // the bodies the plain step deferred (after launch_step_single, same args)
 void launch_step_deferred(const WorldDev& w, const SingleArgs& a, int mode, cudaStream_t st);
+// whole steps of n_worlds small worlds, a cluster each; returns a cudaError_t
+int launch_resident(const WorldDev& w, const ResidentArgs& r, bool uniform, uint32_t n_worlds, uint32_t shared_bytes,
+                    cudaStream_t st);
 void launch_keys_single(const WorldDev& w, const float4* A, int mode, cudaStream_t st);
 void launch_gather_single(const WorldDev& w, const float4* A, const float4* B, const float2* V, float2* pos,
                           float2* pos_old, float2* vel, float2* snap, float v_div, cudaStream_t st);

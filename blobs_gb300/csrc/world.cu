@@ -26,8 +26,8 @@ namespace {
 struct Counters {
   unsigned long long contacts_total[COUNTER_BINS];
   unsigned long long pushouts_total[COUNTER_BINS];
-  uint32_t contacts_sub[COUNTER_BINS];
   unsigned long long defer_total[COUNTER_BINS];
+  uint32_t contacts_sub[COUNTER_BINS];  // (the two cleared together)
   uint32_t defer_sub[COUNTER_BINS];
   uint32_t status;
   uint32_t pad[3];
@@ -199,7 +199,7 @@ struct blobs_world {
   bool multiworld = false, single = false, has_springs = false, has_joints = false, rot_dynamic = false;
   bool any_dynamic = false;
   bool sorted_storage = false;  // single-sphere path: body state in cell-sorted storage (single.cu)
-  int single_mode = 1;          // 0: one uniform world, 1: one world, 2: batched (single.cu)
+  int single_mode = 1;          // 0: one uniform world, 1: one world, 2: batched, 3: batched uniform worlds (single.cu)
   float v_div = 0.0f;           // sorted storage, V untracked: V[vbuf] holds the displacement of a substep of this dt
   int vbuf = 0;                 // sorted storage, V untracked: the V buffer in use
   bool pending = false;
@@ -229,6 +229,14 @@ struct blobs_world {
   Counters* dcounters = nullptr;
   Counters* hcounters = nullptr;  // pinned
   WorldDev dev{};
+  // worlds small enough for the resident kernel, by blocks per world
+  struct ResClass {
+    uint32_t first, count, cluster, shared_bytes;
+  };
+  std::vector<ResClass> res_classes;  // empty: this scene does not take it
+  ResWorld* res_worlds = nullptr;
+  cudaStream_t res_stream[3] = {};    // the classes after the first run beside it
+  cudaEvent_t res_fork = nullptr, res_join[3] = {};
   uint32_t sticky_status = 0;
   std::map<GraphKey, cudaGraphExec_t> graphs;
   std::map<GraphKey, uint32_t> graph_cur_after;  // storage buffer holding the state after the graph
@@ -337,6 +345,14 @@ struct blobs_world {
     arena = nullptr;
     if (hcounters) cudaFreeHost(hcounters);
     hcounters = nullptr;
+    for (int i = 0; i < 3; ++i) {
+      if (res_stream[i]) cudaStreamDestroy(res_stream[i]);
+      if (res_join[i]) cudaEventDestroy(res_join[i]);
+      res_stream[i] = nullptr;
+      res_join[i] = nullptr;
+    }
+    if (res_fork) cudaEventDestroy(res_fork);
+    res_fork = nullptr;
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
     loaded = false;
@@ -354,7 +370,8 @@ struct HostScene {
   std::vector<float> rot, angvel, pend_torque, mass, inertia, gmod, bound_r, col_radius, spr_rest, spr_k, spr_c,
       circles;
   std::vector<uint8_t> bflags, col_sensor;
-  std::vector<uint32_t> body_world, col_world, body_col_start, body_cols, body_spr_start, body_spr, col_parent,
+  std::vector<uint32_t> body_world, col_world, body_col_start, body_cols, body_spr_start, body_spr, spr_bodies, spr_bits,
+      col_parent,
       col_memb, col_filt, spr_a, spr_b, jnt_a, jnt_b;
   std::vector<WorldParam> wparam;
   std::vector<uint32_t> colour_offsets, joint_order;
@@ -694,6 +711,15 @@ int build_host_scene(const blobs_config& cfg, float cell_scale, const blobs_scen
     }
   }
 
+  if (ns) {
+    h.spr_bits.assign((nb + 31) / 32, 0u);
+    for (uint32_t b = 0; b < nb; ++b)
+      if (spr_count[b + 1]) {
+        h.spr_bodies.push_back(b);
+        h.spr_bits[b >> 5] |= 1u << (b & 31u);
+      }
+  }
+
   for (uint32_t j = 0; j < nj; ++j) {
     const uint32_t a = s.jnt_a[j], b = s.jnt_b[j];
     if (a >= nb || b >= nb || a == b) return BLOBS_ERR_INVALID_ARGUMENT;
@@ -800,6 +826,64 @@ int build_host_scene(const blobs_config& cfg, float cell_scale, const blobs_scen
   return BLOBS_OK;
 }
 
+// Which worlds the resident kernel (single.cu) runs, if it is to run this
+// scene: all of them or none.  It is latency that it saves; a batch that
+// fills the GPU is faster through the kernels of a substep, whose blocks keep
+// more warps and more L1.  So its blocks must fit the GPU at once, two to an
+// SM (128 registers), with one body to a thread up to 2,048 bodies a world or
+// two up to 1,024.  Measured, us per step through the kernels -> resident: a
+// world of 300 / 1,000 / 2,000 bodies 101 -> 52, 106 -> 55, 117 -> 74; of
+// 3,000 120 -> 111 sparse but 187 -> 202 crowded, of 4,000 no better; 64
+// worlds of 64 to 2,048 177 -> 110, 256 of 64 to 512 174 -> 98 (two to a
+// thread), 256 of 513 180 -> 203 (512 blocks).
+constexpr uint32_t RES_BLOCKS = 2 * 152;
+constexpr uint32_t RES_LARGEST[RES_PER_THREAD] = {2048u, 1024u};
+
+void resident_classes(const HostScene& h, const blobs_scene& s, uint32_t nw, std::vector<ResWorld>& worlds,
+                      std::vector<blobs_world::ResClass>& classes) {
+  auto body0 = [&](uint32_t k) { return nw > 1 ? s.world_body_offsets[k] : (k ? s.n_bodies : 0u); };
+  uint32_t largest = 0;
+  for (uint32_t k = 0; k < nw; ++k) {
+    largest = std::max(largest, body0(k + 1) - body0(k));
+    if (h.wparam[k].log2w + h.wparam[k].log2h > 30u) return;
+    if ((1u << (h.wparam[k].log2w + h.wparam[k].log2h)) > RES_MAX_CELLS) return;
+  }
+  auto blocks = [](uint32_t n, uint32_t per) {
+    uint32_t c = 1;
+    while (c < RES_MAX_CLUSTER && c * RES_THREADS * per < n) c <<= 1;
+    return c;
+  };
+  uint32_t per = 1;
+  for (; per <= RES_PER_THREAD; ++per) {
+    uint64_t total = 0;
+    for (uint32_t k = 0; k < nw; ++k) total += blocks(body0(k + 1) - body0(k), per);
+    if (largest <= RES_LARGEST[per - 1] && total <= RES_BLOCKS) break;
+  }
+  if (!largest || per > RES_PER_THREAD) return;
+  std::vector<std::pair<uint32_t, uint32_t>> order;  // (blocks, world), most blocks first, then most bodies
+  for (uint32_t k = 0; k < nw; ++k)
+    if (body0(k + 1) > body0(k)) order.push_back({blocks(body0(k + 1) - body0(k), per), k});
+  std::sort(order.begin(), order.end(), [&](const auto& x, const auto& y) {
+    const uint32_t nx = body0(x.second + 1) - body0(x.second), ny = body0(y.second + 1) - body0(y.second);
+    if (x.first != y.first) return x.first > y.first;
+    return nx != ny ? nx > ny : x.second < y.second;
+  });
+  for (const auto& o : order) {
+    const uint32_t k = o.second, b0 = body0(k), b1 = body0(k + 1);
+    ResWorld r{};
+    r.world = k;
+    r.body0 = b0;
+    r.n_bodies = b1 - b0;
+    if (classes.empty() || classes.back().cluster != o.first)
+      classes.push_back({(uint32_t)worlds.size(), 0u, o.first, 0u});
+    classes.back().count += 1;
+    classes.back().shared_bytes =
+        std::max(classes.back().shared_bytes, r.n_bodies * (uint32_t)sizeof(float4) +
+                                                  ((1u << (h.wparam[k].log2w + h.wparam[k].log2h)) + 4u) * 4u);
+    worlds.push_back(r);
+  }
+}
+
 template <class T> cudaError_t up(T* dst, const std::vector<T>& src, cudaStream_t st) {
   if (src.empty()) return cudaSuccess;
   return cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, st);
@@ -808,7 +892,7 @@ template <class T> cudaError_t up(T* dst, const std::vector<T>& src, cudaStream_
 // Lay out (or size) every device array of the scene.
 void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const HostScene& h, uint32_t nb, uint32_t nc,
            uint32_t ns, uint32_t nj, uint32_t nw, uint32_t ncirc, uint32_t n_cells, uint32_t n_tiles,
-           bool sorted_storage) {
+           bool sorted_storage, const std::vector<ResWorld>& res, ResWorld** res_worlds) {
   const uint32_t ss = sorted_storage ? nb : 0u;
   d.sa[0] = cv.take<float4>(ss);
   d.sa[1] = cv.take<float4>(ss);
@@ -843,6 +927,8 @@ void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const Hos
   d.body_cols = cv.take<uint32_t>(nc);
   d.body_spr_start = cv.take<uint32_t>(nb + 1);
   d.body_spr = cv.take<uint32_t>(2 * (size_t)ns);
+  d.spr_bodies = cv.take<uint32_t>(sorted_storage ? h.spr_bodies.size() : 0u);
+  d.spr_bits = cv.take<uint32_t>(sorted_storage ? h.spr_bits.size() : 0u);
   d.col_parent = cv.take<uint32_t>(nc);
   d.col_off = cv.take<float2>(nc);
   d.col_radius = cv.take<float>(nc);
@@ -869,6 +955,10 @@ void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const Hos
   d.wparam = cv.take<WorldParam>(nw);
   d.cell_count = cv.take<uint32_t>(n_cells);
   d.cell_start = cv.take<uint32_t>((size_t)n_cells + 1);
+  d.cell_count_b = cv.take<uint32_t>(res.empty() ? 0u : 2 * (size_t)n_cells);
+  d.key_b = cv.take<uint32_t>(res.empty() ? 0u : ss);
+  d.rank_b = cv.take<uint32_t>(res.empty() ? 0u : ss);
+  *res_worlds = cv.take<ResWorld>(res.size());
   d.rank = cv.take<uint32_t>(nc);
   d.sorted = cv.take<float4>(sorted_storage ? 0u : nc);
   d.clist = cv.take<Contact>(sorted_storage ? 0u : (size_t)nc * CL_CAP);
@@ -907,6 +997,65 @@ void mark_end(blobs_world* w) {
   else cudaEventRecord(b, w->st());
 }
 
+// Does the resident kernel run this world's steps?  Not with phase
+// timing (its phases are kernels), the event stream (ordered by substep over
+// all worlds) or the recording of contacts.
+bool takes_resident(const blobs_world* w) {
+  return !w->res_classes.empty() && w->cfg.collisions_enabled && !w->timing && !w->events_on && !w->rec_list;
+}
+
+// `n_steps` steps of every world by the resident kernel, at most
+// RES_LAUNCH_STEPS of them to a launch.
+constexpr uint32_t RES_LAUNCH_STEPS = 64;
+
+cudaError_t enqueue_resident(blobs_world* w, float dt, float old_dt, bool pending, uint32_t n_steps) {
+  const WorldDev& d = w->dev;
+  cudaStream_t st = w->st();
+  if (!w->keys_valid) {
+    launch_keys_single(d, d.sa[w->cur], w->single_mode, st);
+    w->enqueued += 1;
+    w->keys_valid = true;
+  }
+  cudaError_t e = cudaSuccess;
+  const size_t n_class = w->res_classes.size();
+  for (uint32_t done = 0; done < n_steps && e == cudaSuccess;) {
+    const uint32_t steps = std::min(n_steps - done, RES_LAUNCH_STEPS);
+    e = cudaMemsetAsync(d.contacts_sub, 0, 2 * sizeof(uint32_t) * COUNTER_BINS, st);  // and defer_sub
+    ResidentArgs r;
+    std::memset(&r, 0, sizeof(r));
+    r.base.dt = dt;
+    r.base.ratio_first = done ? dt / dt : dt / old_dt;
+    r.base.ratio_rest = dt / dt;
+    r.base.pending = pending && !done ? 1u : 0u;
+    r.base.springs = w->has_springs ? 1u : 0u;
+    r.base.rot_dynamic = w->rot_dynamic ? 1u : 0u;
+    r.base.move_v = r.base.v_vel = w->v_tracks() ? 1u : 0u;
+    r.base.mass4r = w->mass4r ? 1u : 0u;
+    r.base.contacts = r.base.do_keys = 1u;
+    r.n_steps = steps;
+    r.substeps = w->cfg.substeps;
+    r.cur = w->cur;
+    r.vbuf = (uint32_t)w->vbuf;
+    const bool uniform = w->single_mode == 0 || w->single_mode == 3;
+    if (n_class > 1 && e == cudaSuccess) e = cudaEventRecord(w->res_fork, st);
+    for (size_t k = 0; k < n_class && e == cudaSuccess; ++k) {
+      const auto& c = w->res_classes[k];
+      cudaStream_t s = k ? w->res_stream[k - 1] : st;
+      if (k) e = cudaStreamWaitEvent(s, w->res_fork, 0);
+      r.worlds = w->res_worlds + c.first;
+      r.cluster = c.cluster;
+      if (e == cudaSuccess) e = (cudaError_t)launch_resident(d, r, uniform, c.count, c.shared_bytes, s);
+      if (k && e == cudaSuccess) e = cudaEventRecord(w->res_join[k - 1], s);
+      w->enqueued += 1;
+    }
+    for (size_t k = 1; k < n_class && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(st, w->res_join[k - 1], 0);
+    if (steps % 2 && w->cfg.substeps % 2 == 0) w->cur ^= 1u;  // each step's first substep moves the storage back
+    done += steps;
+  }
+  if (!w->v_tracks()) w->v_div = dt;
+  return e;
+}
+
 void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool first_in_step, bool last_in_step) {
   const WorldDev& d = w->dev;
   float2* in = w->pos[w->cur];
@@ -931,6 +1080,11 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     const int cur = (int)w->cur;
     SingleArgs a;
     std::memset(&a, 0, sizeof(a));
+    a.cell_start = d.cell_start;
+    a.cell_count = d.cell_count;
+    a.key_out = d.key;
+    a.rank_out = d.rank;
+    a.wparam = d.wparam;
     a.dt = dt;
     a.ratio_first = dt / old_dt;
     a.ratio_rest = dt / dt;
@@ -967,7 +1121,10 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
         a.cand = d.sa[in];
         a.own_cell = d.ckey;
       } else {
-        launch_scatter_cand(d, d.sa[cur], d.cand, st);
+        a.a_in = d.sa[cur];
+        a.b_in = d.sb[cur];
+        a.v_in = d.sv[cur];  // springs: tracked with the state
+        launch_scatter_cand(d, a, d.cand, st);
         a.cand = d.cand;
         a.own_cell = d.key;
       }
@@ -986,6 +1143,11 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     a.a_out = d.sa[out];
     a.b_out = d.sb[out];
     a.v_out = d.sv[w->v_tracks() ? out : w->vbuf];
+    if (a.springs && (first_in_step || !coll)) {
+      // (the other substeps' forces come with the scatter)
+      launch_springs(d, a, st);
+      w->enqueued += 1;
+    }
     mark_begin(w, coll ? PHASE_CONTACT : PHASE_INTEGRATE);
     launch_step_single(d, a, w->single_mode, st);
     if (coll) {
@@ -1052,13 +1214,20 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
 
 // One reference `integrate(substeps, delta)` (physics.rs:397-422) enqueued
 // eagerly, honouring pending requests and the old_dt ratio.
-void enqueue_integrate(blobs_world* w, float delta) {
+cudaError_t enqueue_integrate(blobs_world* w, float delta) {
   const float step_delta = delta / (float)w->cfg.substeps;
+  if (takes_resident(w)) {
+    const cudaError_t e = enqueue_resident(w, step_delta, w->old_dt, w->pending, 1);
+    w->pending = false;
+    if (w->any_dynamic) w->old_dt = step_delta;
+    return e;
+  }
   for (uint32_t s = 0; s < w->cfg.substeps; ++s) {
     enqueue_substep(w, step_delta, w->old_dt, w->pending, s == 0, s + 1 == w->cfg.substeps);
     w->pending = false;
     if (w->any_dynamic) w->old_dt = step_delta;
   }
+  return cudaSuccess;
 }
 
 uint32_t f2bits(float f) {
@@ -1088,15 +1257,24 @@ int launch_steady(blobs_world* w, float delta, uint32_t n_steps) {
     w->capturing = true;
     w->recording = w->timing ? &w->graph_timing[key] : nullptr;
     const uint64_t before = w->enqueued;
-    for (uint32_t n = 0; n < n_steps; ++n)
-      for (uint32_t s = 0; s < w->cfg.substeps; ++s)
-        enqueue_substep(w, step_delta, step_delta, false, s == 0, s + 1 == w->cfg.substeps);
+    cudaError_t queued = cudaSuccess;
+    if (takes_resident(w)) {
+      queued = enqueue_resident(w, step_delta, step_delta, false, n_steps);
+    } else {
+      for (uint32_t n = 0; n < n_steps; ++n)
+        for (uint32_t s = 0; s < w->cfg.substeps; ++s)
+          enqueue_substep(w, step_delta, step_delta, false, s == 0, s + 1 == w->cfg.substeps);
+    }
     w->capturing = false;
     w->recording = nullptr;
     w->graph_kernels[key] = w->enqueued - before;
     w->graph_cur_after[key] = w->cur;
     w->enqueued = before;
     e = cudaStreamEndCapture(w->st(), &g);
+    if (e == cudaSuccess && queued != cudaSuccess) {
+      cudaGraphDestroy(g);
+      e = queued;
+    }
     if (e != cudaSuccess) {
       w->cur = cur0;  // nothing ran
       return blobs_map_cuda(e);
@@ -1138,7 +1316,8 @@ int run_steps(blobs_world* w, double delta, uint32_t n_steps) {
         w->launched_sets.push_back(w->recording);
     }
     const uint64_t before = w->enqueued;
-    enqueue_integrate(w, df);
+    e = enqueue_integrate(w, df);
+    if (e != cudaSuccess) return blobs_map_cuda(e);
     w->kernels_launched += w->enqueued - before;
     w->recording = nullptr;
     w->time += delta;
@@ -1439,25 +1618,30 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   bool mass4r = sorted_storage;  // rigid_body.rs:96-128 with one collider, no override: m = 4 r
   for (uint32_t i = 0; i < nb && mass4r; ++i) mass4r = h.mass[i] == h.col_radius[i] * 4.0f;
   w->mass4r = mass4r;
-  bool uniform = sorted_storage && nw == 1;
-  uint32_t first_dyn = 0xffffffffu;
-  for (uint32_t i = 0; i < nb && uniform; ++i) {
-    if (h.bflags[i] & BF_STATIC) uniform = false;
-    if (h.gmod[i] != h.gmod[0] || std::isnan(h.gmod[i])) uniform = false;
-    if (!(h.mass[i] == h.col_radius[i] * 4.0f) || !(h.bound_r[i] == h.col_radius[i])) uniform = false;
-    if ((h.bflags[i] & BF_FIRST_DYN) && first_dyn == 0xffffffffu) first_dyn = i;
+  // and neither does a batch of such worlds
+  bool uniform = mass4r;
+  for (uint32_t k = 0; k < nw && uniform; ++k) {
+    const uint32_t b0 = nw > 1 ? scene->world_body_offsets[k] : 0u, b1 = nw > 1 ? scene->world_body_offsets[k + 1] : nb;
+    uint32_t first_dyn = 0xffffffffu;
+    for (uint32_t i = b0; i < b1 && uniform; ++i) {
+      if (h.bflags[i] & BF_STATIC) uniform = false;
+      if (h.gmod[i] != h.gmod[b0] || std::isnan(h.gmod[i])) uniform = false;
+      if (!(h.bound_r[i] == h.col_radius[i])) uniform = false;
+      if ((h.bflags[i] & BF_FIRST_DYN) && first_dyn == 0xffffffffu) first_dyn = i;
+    }
+    h.wparam[k].first_dyn = first_dyn;
+    h.wparam[k].uniform_gmod = b1 > b0 ? h.gmod[b0] : 1.0f;
   }
-  if (!h.wparam.empty()) {
-    h.wparam[0].first_dyn = first_dyn;
-    h.wparam[0].uniform_gmod = nb ? h.gmod[0] : 1.0f;
-  }
-  carve(sizer, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage);
+  std::vector<ResWorld> res;
+  w->res_classes.clear();
+  if (sorted_storage && nc) resident_classes(h, *scene, nw, res, w->res_classes);
+  carve(sizer, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds);
   e = device_alloc(w->cfg.device, &w->arena, sizer.off + 256);
   if (e != cudaSuccess) return blobs_map_cuda(e);
   w->arena_bytes = sizer.off + 256;
   Carver cv;
   cv.base = static_cast<char*>(w->arena);
-  carve(cv, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage);
+  carve(cv, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds);
   d.n_bodies = nb;
   d.n_cols = nc;
   d.n_springs = ns;
@@ -1498,6 +1682,11 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   UP(d.body_cols, h.body_cols);
   UP(d.body_spr_start, h.body_spr_start);
   UP(d.body_spr, h.body_spr);
+  if (sorted_storage) {
+    UP(d.spr_bodies, h.spr_bodies);
+    UP(d.spr_bits, h.spr_bits);
+    d.n_spr_bodies = (uint32_t)h.spr_bodies.size();
+  }
   UP(d.col_parent, h.col_parent);
   UP(d.col_off, h.col_off);
   UP(d.col_radius, h.col_radius);
@@ -1522,6 +1711,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   UP(d.jnt_local, h.jnt_local);
   UP(d.circles, h.circles);
   UP(d.wparam, h.wparam);
+  UP(w->res_worlds, res);
 #undef UP
   std::vector<float4> sa, sb, sc;
   std::vector<uint32_t> ident;
@@ -1551,6 +1741,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
     if (e == cudaSuccess) e = up(d.where, ident, s);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_count, 0, sizeof(uint32_t) * (size_t)h.n_cells, s);
+  if (e == cudaSuccess && !res.empty()) e = cudaMemsetAsync(d.cell_count_b, 0, 2 * sizeof(uint32_t) * (size_t)h.n_cells, s);
   if (e == cudaSuccess && !sorted_storage) e = cudaMemsetAsync(d.bslow, 0, nb, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(Counters), s);
   if (e == cudaSuccess && sorted_storage) e = cudaMemsetAsync(d.defer_count, 0, sizeof(uint32_t), s);
@@ -1558,6 +1749,18 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
     cudaFree(w->arena);
     w->arena = nullptr;
     return blobs_map_cuda(e);
+  }
+  if (w->res_classes.size() > 1 && !w->res_join[2]) {
+    e = w->res_fork ? cudaSuccess : cudaEventCreateWithFlags(&w->res_fork, cudaEventDisableTiming);
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
+      if (!w->res_stream[i]) e = cudaStreamCreateWithFlags(&w->res_stream[i], cudaStreamNonBlocking);
+      if (e == cudaSuccess && !w->res_join[i]) e = cudaEventCreateWithFlags(&w->res_join[i], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) {
+      cudaFree(w->arena);
+      w->arena = nullptr;
+      return blobs_map_cuda(e);
+    }
   }
   w->dev = d;
   w->attach_events();
@@ -1575,7 +1778,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   w->multiworld = nw > 1;
   w->single = h.single;
   w->sorted_storage = sorted_storage;
-  w->single_mode = nw > 1 ? 2 : (uniform ? 0 : 1);
+  w->single_mode = nw > 1 ? (uniform ? 3 : 2) : (uniform ? 0 : 1);
   w->v_div = 0.0f;
   w->vbuf = 0;
   w->has_springs = ns > 0;

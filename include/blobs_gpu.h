@@ -204,7 +204,10 @@ int blobs_world_kernel_launches(blobs_world* w, uint64_t* count);
 
 /* enabled = 1: CUDA events are recorded around each kernel phase of every
  * substep (inside the step graphs); 2: around the contact phase only (its
- * kernel timed without event nodes between the other kernels); 0: off. */
+ * kernel timed without event nodes between the other kernels); 0: off.
+ * Worlds that would otherwise run whole steps in one kernel (up to 2,048
+ * single spheres) are stepped phase by phase while timing is on; the results
+ * are the same. */
 int blobs_world_set_timing(blobs_world* w, int enabled);
 /* Device milliseconds and launch counts per phase since the previous call:
  * [0] cell scan, [1] scatter + forces, [2] contacts (+ fused integration),
@@ -228,7 +231,7 @@ int blobs_world_pushout_count(blobs_world* w, uint64_t* total);
 /* No counterpart in the reference (a cost diagnostic): bodies of the
  * single-sphere path whose 3x3 cells held more than 64 candidates, or which
  * had more near candidates than the step kernel takes (32 in the plain step
- * of a uniform world, 12 otherwise), and whose contacts were therefore
+ * of uniform worlds, 12 otherwise), and whose contacts were therefore
  * resolved by a warp of their own -- since load and in the last substep. */
 int blobs_world_deferred_count(blobs_world* w, uint64_t* total, uint64_t* last_substep);
 /* The broadphase output for the current collider snapshots: every collider
