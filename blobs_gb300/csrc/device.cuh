@@ -110,6 +110,12 @@ struct WorldDev {
   uint32_t* jb_joint_start;
   uint32_t* jb_body_start;
   uint32_t* jb_bodies;
+  // the solves (joint, iteration) of a block's joints over JB_ITERS
+  // iterations, level by level: block k's are jb_op[JB_ITERS * (its first
+  // joint) ..], its levels' bounds jb_level[jb_level_start[k] .. jb_level_start[k+1])
+  uint16_t* jb_op;
+  uint16_t* jb_level;
+  uint32_t* jb_level_start;
   uint32_t n_jblocks;
 
   float* circles;            // 3 per circle
@@ -352,7 +358,7 @@ constexpr int CONTACT_LIST = 24;           // per-body sorted contact list kept 
 constexpr uint32_t CL_CAP = 8;             // general path: contacts kept per collider
 constexpr uint32_t COUNTER_BINS = 64;
 constexpr uint32_t REC_CAP = 16;           // recorded contacts per body and substep (adjoint)
-constexpr int JB_THREADS = 128;            // k_joint_blocks: one thread per small component
+constexpr int JB_THREADS = 128;            // k_joint_blocks: threads of a block, and small components at most
 constexpr uint32_t RES_THREADS = 256;      // resident kernel: threads of a block,
 constexpr uint32_t RES_PER_THREAD = 2;     // bodies of a thread at most,
 constexpr uint32_t RES_MAX_CLUSTER = 8;    // blocks of a world at most,
@@ -361,7 +367,9 @@ constexpr uint32_t RES_MAX_CELLS = 2 * RES_MAX_BODIES;  // and cells (what the g
 constexpr uint32_t JB_MAX_JOINTS = 64;     // larger components take the coloured sweep
 constexpr uint32_t JB_JOINTS = 512;        // joints staged in shared memory per block
 constexpr uint32_t JB_BODIES = 640;        // bodies staged per block (<= JB_JOINTS + JB_THREADS)
-constexpr uint32_t JB_ITERS = 4;           // iterations whose rotation terms a block keeps
+constexpr uint32_t JB_ITERS = 4;           // iterations whose solves a block lays out in levels
+constexpr uint32_t JB_OP_BITS = 10;        // bits of a solve's joint (< JB_JOINTS), the iteration above them
+constexpr uint32_t JB_MAX_LEVELS = JB_ITERS * JB_MAX_JOINTS;  // a component's solves one after the other
 constexpr uint32_t JL_STATIC_A = 1u << 15; // jnt_local flags: body a / b is static
 constexpr uint32_t JL_STATIC_B = 1u << 31;
 
