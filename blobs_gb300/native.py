@@ -500,13 +500,15 @@ class SpatialHash:
         nq = len(qradius)
         offsets = np.zeros(nq + 1, np.uint64)
         total = ctypes.c_uint64()
-        if cap is None:
-            st = lib().blobs_spatial_hash_query(self._h, nq, _ptr(qxy), _ptr(qradius), _ptr(offsets), None, 0,
-                                                ctypes.byref(total))
-            if st not in (OK, ERR_OVERFLOW):
-                check(st, "blobs_spatial_hash_query")
-            cap = int(total.value)
-        ids = np.zeros(max(cap, 1), np.uint64)
-        check(lib().blobs_spatial_hash_query(self._h, nq, _ptr(qxy), _ptr(qradius), _ptr(offsets), _ptr(ids), cap,
-                                             ctypes.byref(total)), "blobs_spatial_hash_query")
+        # without a capacity: room for 16 results a query (untouched pages cost nothing), and a second call where
+        # there are more
+        room = cap if cap is not None else 16 * nq + 1024
+        ids = np.empty(max(room, 1), np.uint64)
+        st = lib().blobs_spatial_hash_query(self._h, nq, _ptr(qxy), _ptr(qradius), _ptr(offsets), _ptr(ids), room,
+                                            ctypes.byref(total))
+        if st == ERR_OVERFLOW and cap is None and total.value > room:
+            ids = np.empty(int(total.value), np.uint64)
+            st = lib().blobs_spatial_hash_query(self._h, nq, _ptr(qxy), _ptr(qradius), _ptr(offsets), _ptr(ids),
+                                                int(total.value), ctypes.byref(total))
+        check(st, "blobs_spatial_hash_query")
         return offsets, ids[:int(total.value)]
