@@ -171,12 +171,7 @@ __device__ __forceinline__ void single_event(const WorldDev& w, const SingleArgs
 // (sub: the substep's own counts too)
 __device__ __forceinline__ void count_warp(const WorldDev& w, uint32_t ncontacts, uint32_t npush, bool deferred,
                                            bool sub) {
-  uint32_t t = ncontacts, p = npush;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    t += __shfl_xor_sync(0xffffffffu, t, o);
-    p += __shfl_xor_sync(0xffffffffu, p, o);
-  }
+  const uint32_t t = __reduce_add_sync(0xffffffffu, ncontacts), p = __reduce_add_sync(0xffffffffu, npush);
   const uint32_t nw = __popc(__ballot_sync(0xffffffffu, deferred));
   if ((threadIdx.x & 31u) == 0u) {
     const uint32_t bin = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) & (COUNTER_BINS - 1);
@@ -484,9 +479,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
   for (uint32_t base = 0; base < total;) {
     // this round: the ranges that lie wholly in [base, base + PAIR_CAP)
     const bool mine = kk > 0u && off >= base && off + kk <= base + PAIR_CAP;
-    uint32_t end = mine ? off + kk : base;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) end = max(end, __shfl_xor_sync(0xffffffffu, end, o));
+    const uint32_t end = __reduce_max_sync(0xffffffffu, mine ? off + kk : base);
     const uint32_t cnt = end - base, r0 = off - base;
     if (mine) {
       uint32_t e = r0;
