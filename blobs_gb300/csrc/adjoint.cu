@@ -13,16 +13,20 @@
 // p_c - v0 dt (physics.rs:334-336), so disp = v0 dt ratio.  Push-out
 // contacts are discrete events and are not differentiated.
 //
-// Three kernels per substep, in order:
-//   k_adj_body    per body: Verlet, clamp mask, velocity request -> the
+// Three parts per substep, in order:
+//   body          per body: Verlet, clamp mask, velocity request -> the
 //                 adjoints of p_c and a, the outgoing adjoint of po
 //   k_adj_springs per spring: Jacobians of the (quirky) spring force ->
 //                 the adjoints of the spring's d = pb - pa and rv = va - vb,
 //                 and dL/dk
-//   k_adj_gather  per body: its recorded contacts (the Jacobian of the
+//   gather        per body: its recorded contacts (the Jacobian of the
 //                 mass-ratio correction, each pair evaluated from both
 //                 sides) -> the adjoint of its snapshot; its springs ->
 //                 the adjoints of its position and velocity
+// The gather of a substep and the body part of the one before it are one
+// kernel (k_adj_gather): a body's outgoing adjoints go on in registers, and a
+// substep is two launches.  The parts read few bytes in short dependent
+// chains; launches and first loads bound them.
 // Every sum runs in a fixed order (ascending partner id, ascending spring
 // index), so the gradients are deterministic: no float atomics.
 #include "device.cuh"
@@ -30,10 +34,9 @@
 
 namespace blobs {
 
-__global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) {
-  pdl_enter();
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= w.n_bodies) return;
+// The body part: from the adjoints of (p', po', s', v').
+__device__ __forceinline__ void adj_body(const WorldDev& w, const AdjointSubstep& a, uint32_t b, float2 lp1, float2 lpo1,
+                                         float2 ls1, float2 lv1) {
   const uint8_t fl = w.bflags[b];
   const float dt = a.dt;
   // clamp mask of the wall extension: the derivative passes where the body
@@ -46,7 +49,6 @@ __global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) 
     mask.x = (s1.x > wp.box_lo_x + br && s1.x < wp.box_hi_x - br) ? 1.0f : 0.0f;
     mask.y = (s1.y > wp.box_lo_y + br && s1.y < wp.box_hi_y - br) ? 1.0f : 0.0f;
   }
-  const float2 lp1 = a.lp_in[b], lpo1 = a.lpo_in[b], ls1 = a.ls_in[b], lv1 = a.lv_in[b];
   const float2 lpnew = v2(ls1.x + mask.x * lp1.x, ls1.y + mask.y * lp1.y);
   float2 lpc, la = v2(0.0f, 0.0f), lpo = v2(0.0f, 0.0f);
   if (fl & BF_STATIC) {
@@ -69,6 +71,12 @@ __global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) 
   a.lpc[b] = lpc;
   a.la[b] = la;
   a.lpo_out[b] = lpo;
+}
+
+__global__ void __launch_bounds__(256) k_adj_body(WorldDev w, AdjointSubstep a) {
+  pdl_enter();
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < w.n_bodies) adj_body(w, a, b, a.lp_in[b], a.lpo_in[b], a.ls_in[b], a.lv_in[b]);
 }
 
 __global__ void __launch_bounds__(256) k_adj_springs(WorldDev w, AdjointSubstep a) {
@@ -120,7 +128,12 @@ __global__ void __launch_bounds__(256) k_adj_springs(WorldDev w, AdjointSubstep 
   a.spr_terms[sidx] = make_float4(ldx, ldy, lrvx, lrvy);
 }
 
-__global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a) {
+// The gather of substep a, then the body part of the substep before it.
+// (lpc alternates between the two: the gather reads its partners' values
+// while other bodies write theirs for the substep before.  Without one the
+// adjoints are written out.)
+template <bool BEFORE>
+__global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a, AdjointSubstep before) {
   pdl_enter();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= w.n_bodies) return;
@@ -155,7 +168,6 @@ __global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a
     const float gx = jxx * ux + jxy * uy, gy = jxy * ux + jyy * uy;
     ls = hi ? v2(ls.x + gx, ls.y + gy) : v2(ls.x - gx, ls.y - gy);
   }
-  a.ls_out[c] = ls;
   // springs, ascending spring index: p_c = p + corrections(s), so the
   // position adjoint is lpc plus the spring terms
   float2 lp = a.lpc[c], lv = v2(0.0f, 0.0f);
@@ -173,15 +185,25 @@ __global__ void __launch_bounds__(256) k_adj_gather(WorldDev w, AdjointSubstep a
       }
     }
   }
-  a.lp_out[c] = lp;
-  a.lv_out[c] = lv;
+  if (BEFORE) {
+    adj_body(w, before, c, lp, a.lpo_out[c], ls, lv);
+  } else {
+    a.lp_out[c] = lp;
+    a.ls_out[c] = ls;
+    a.lv_out[c] = lv;
+  }
 }
 
-void launch_adjoint_substep(const WorldDev& w, const AdjointSubstep& a, cudaStream_t st) {
+void launch_adjoint_body(const WorldDev& w, const AdjointSubstep& a, cudaStream_t st) {
+  if (w.n_bodies) launch_pdl(k_adj_body, (w.n_bodies + 255u) / 256u, 256, st, true, w, a);
+}
+
+void launch_adjoint_substep(const WorldDev& w, const AdjointSubstep& a, const AdjointSubstep* before, cudaStream_t st) {
   if (!w.n_bodies) return;
-  launch_pdl(k_adj_body, (w.n_bodies + 255u) / 256u, 256, st, true, w, a);
   if (w.n_springs) launch_pdl(k_adj_springs, (w.n_springs + 255u) / 256u, 256, st, true, w, a);
-  launch_pdl(k_adj_gather, (w.n_bodies + 255u) / 256u, 256, st, true, w, a);
+  const uint32_t g = (w.n_bodies + 255u) / 256u;
+  if (before) launch_pdl(k_adj_gather<true>, g, 256, st, true, w, a, *before);
+  else launch_pdl(k_adj_gather<false>, g, 256, st, true, w, a, a);
 }
 
 }  // namespace blobs

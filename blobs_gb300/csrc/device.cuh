@@ -315,6 +315,10 @@ struct SingleArgs {
   uint32_t* rec_list;
   uint32_t* rec_n;
   uint32_t* rec_max;
+  // and with it the state after the substep, arena order (rec_v in worlds that track V)
+  float2* rec_p;
+  float2* rec_s;
+  float2* rec_v;
 };
 
 // A world of the resident kernel: its bodies are storage slots

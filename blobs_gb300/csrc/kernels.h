@@ -91,7 +91,6 @@ struct AdjointSubstep {
   const float2* p_t;
   const float2* s_t;
   const float2* v_t;
-  const float2* p_t1;
   const float2* s_t1;
   const uint32_t* rec_list;  // contacts of each body in the substep, as recorded (REC_CAP x n_bodies)
   const uint32_t* rec_n;     // per body: recorded contacts
@@ -114,6 +113,10 @@ struct AdjointSubstep {
   uint32_t first_substep;  // the rollout's first substep (dt / old_dt applies)
   uint32_t vreq_pending;   // velocity requests were pending at the rollout's start
 };
-void launch_adjoint_substep(const WorldDev& w, const AdjointSubstep& a, cudaStream_t st);
+// the body part of a substep alone
+void launch_adjoint_body(const WorldDev& w, const AdjointSubstep& a, cudaStream_t st);
+// the spring and gather parts of a substep whose body part is done, and the
+// body part of the substep before it (NULL: there is none)
+void launch_adjoint_substep(const WorldDev& w, const AdjointSubstep& a, const AdjointSubstep* before, cudaStream_t st);
 
 }  // namespace blobs

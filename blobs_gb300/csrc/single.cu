@@ -297,7 +297,7 @@ struct DeferWarp {
 // gravity (and the spring forces found before the contacts), Verlet, the
 // snapshot, the constraints, and the next substep's cell key and rank.  p is
 // the position after the contacts.
-template <int MODE>
+template <int MODE, bool HOOKS>
 __device__ __forceinline__ void finish_single(const WorldDev& w, const SingleArgs& a, const WorldParam& wp,
                                               const BodyConst& k, uint32_t j, uint32_t c, float4 av, float4 bv,
                                               float2 p) {
@@ -351,6 +351,11 @@ __device__ __forceinline__ void finish_single(const WorldDev& w, const SingleArg
   a.a_out[j] = make_float4(snap.x, snap.y, r, av.w);
   a.b_out[j] = make_float4(p.x, p.y, po.x, po.y);
   if (a.v_vel || a.write_v) a.v_out[j] = vel;
+  if (HOOKS && a.rec_p) {  // the state after the substep for the adjoint, arena order
+    a.rec_p[c] = p;
+    a.rec_s[c] = snap;
+    if (a.v_vel) a.rec_v[c] = vel;
+  }
   if (a.do_keys) {
     const uint32_t key = cell_key(wp, snap);
     a.key_out[j] = key;
@@ -763,7 +768,7 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
         a.rec_n[c] = nrec;
         if (nrec) atomicMax(a.rec_max, nrec);
       }
-      finish_single<MODE>(w, a, wp, k, j, c, av, bv, p);
+      finish_single<MODE, HOOKS>(w, a, wp, k, j, c, av, bv, p);
     }
   }
   if (WARP2) {
@@ -774,7 +779,7 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
     // the records again (cache hits) rather than registers held across
     // phase 2
     if (MODE == 3 && live) wp0 = a.wparam[slot_world<MODE>(w, j)];
-    if (live && !deferred) finish_single<MODE>(w, a, wp0, k, j, c, a.a_in[j], a.b_in[j], p);
+    if (live && !deferred) finish_single<MODE, HOOKS>(w, a, wp0, k, j, c, a.a_in[j], a.b_in[j], p);
   }
   return deferred;
 }
@@ -966,7 +971,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
         a.rec_n[c] = nrec;
         if (nrec) atomicMax(a.rec_max, nrec);
       }
-      finish_single<MODE>(w, a, wp, k, j, c, av, bv, p);
+      finish_single<MODE, HOOKS>(w, a, wp, k, j, c, av, bv, p);
     }
   } else if (lane == 0) {
     uint32_t nc = 0, np = 0, nr = 0;
@@ -977,7 +982,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
       a.rec_n[c] = nr;
       if (nr) atomicMax(a.rec_max, nr);
     }
-    finish_single<MODE>(w, a, wp, k, j, c, av, bv, p);
+    finish_single<MODE, HOOKS>(w, a, wp, k, j, c, av, bv, p);
   }
   __syncwarp();
 }
@@ -1141,6 +1146,14 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentAr
       a.cell_count = count_next;
       a.key_out = key_next;
       a.rank_out = rnk_next;
+      if (HOOKS) {  // a substep's records follow those of the one before
+        a.rec_list = r.base.rec_list + (size_t)REC_CAP * w.n_bodies * sub;
+        a.rec_n = r.base.rec_n + (size_t)w.n_bodies * sub;
+        a.rec_max = r.base.rec_max + sub;
+        a.rec_p = r.base.rec_p + (size_t)w.n_bodies * sub;
+        a.rec_s = r.base.rec_s + (size_t)w.n_bodies * sub;
+        a.rec_v = r.base.rec_v + (size_t)w.n_bodies * sub;
+      }
       s_ndef = 0u;
     }
     // ---- cell table and candidates (block_scan's barriers publish the arguments)
@@ -1377,7 +1390,8 @@ void launch_step_deferred(const WorldDev& w, const SingleArgs& a, int mode, cuda
 int launch_resident(const WorldDev& w, const ResidentArgs& r, bool uniform, uint32_t n_worlds, uint32_t shared_bytes,
                     cudaStream_t st) {
   if (!n_worlds) return 0;
-  auto kernel = uniform ? k_resident<0, false> : k_resident<1, false>;
+  auto kernel = r.base.rec_list ? (uniform ? k_resident<0, true> : k_resident<1, true>)
+                                : (uniform ? k_resident<0, false> : k_resident<1, false>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(RES_MAX_BODIES * sizeof(float4) + (RES_MAX_CELLS + 4u) * sizeof(uint32_t)));
   if (e != cudaSuccess) return (int)e;

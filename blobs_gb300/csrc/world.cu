@@ -250,6 +250,7 @@ struct blobs_world {
   uint32_t* rec_list = nullptr;
   uint32_t* rec_n = nullptr;
   uint32_t* rec_max = nullptr;
+  float2 *rec_p = nullptr, *rec_s = nullptr, *rec_v = nullptr;
   // differentiable rollout: checkpoints of the arena-order state
   struct Recording {
     bool valid = false;
@@ -1046,10 +1047,10 @@ void mark_end(blobs_world* w) {
 }
 
 // Does the resident kernel run this world's steps?  Not with phase
-// timing (its phases are kernels), the event stream (ordered by substep over
-// all worlds) or the recording of contacts.
+// timing (its phases are kernels) or the event stream (ordered by substep over
+// all worlds); the reverse pass's recomputation records no events.
 bool takes_resident(const blobs_world* w) {
-  return !w->res_classes.empty() && w->cfg.collisions_enabled && !w->timing && !w->events_on && !w->rec_list;
+  return !w->res_classes.empty() && w->cfg.collisions_enabled && !w->timing && (!w->events_on || w->rec_list);
 }
 
 // `n_steps` steps of every world by the resident kernel, at most
@@ -1080,6 +1081,15 @@ cudaError_t enqueue_resident(blobs_world* w, float dt, float old_dt, bool pendin
     r.base.move_v = r.base.v_vel = w->v_tracks() ? 1u : 0u;
     r.base.mass4r = w->mass4r ? 1u : 0u;
     r.base.contacts = r.base.do_keys = 1u;
+    if (w->rec_list) {  // of the first substep; the others' follow
+      const size_t at = (size_t)done * w->cfg.substeps;
+      r.base.rec_list = w->rec_list + (size_t)REC_CAP * w->nb * at;
+      r.base.rec_n = w->rec_n + (size_t)w->nb * at;
+      r.base.rec_max = w->rec_max + at;
+      r.base.rec_p = w->rec_p + (size_t)w->nb * at;
+      r.base.rec_s = w->rec_s + (size_t)w->nb * at;
+      r.base.rec_v = w->rec_v + (size_t)w->nb * at;
+    }
     r.n_steps = steps;
     r.substeps = w->cfg.substeps;
     r.cur = w->cur;
@@ -1146,6 +1156,9 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     a.rec_list = w->rec_list;
     a.rec_n = w->rec_n;
     a.rec_max = w->rec_max;
+    a.rec_p = w->rec_p;
+    a.rec_s = w->rec_s;
+    a.rec_v = w->rec_v;
     int in = cur, out = cur ^ 1;
     if (coll) {
       if (!w->keys_valid) {
@@ -2226,7 +2239,7 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
   // scratch of the reverse pass: sized by a first carve, then carved
   const size_t slice = nb * sizeof(float2);
   struct Scratch {
-    float2 *sp, *ss, *sv, *adj[2][4], *lpc, *la, *lv0;
+    float2 *sp, *ss, *sv, *adj[2][4], *lpc[2], *la, *lv0;
     uint32_t* rec_list;
     uint32_t* rec_n;
     uint32_t* rec_max;
@@ -2244,7 +2257,7 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
     x.spr_terms = cv.take<float4>(w->ns ? w->ns : 1);
     for (int k = 0; k < 2; ++k)
       for (int m = 0; m < 4; ++m) x.adj[k][m] = cv.take<float2>(nb);  // adjoints of (p, po, s, v) in / out
-    x.lpc = cv.take<float2>(nb);
+    for (int k = 0; k < 2; ++k) x.lpc[k] = cv.take<float2>(nb);
     x.la = cv.take<float2>(nb);
     x.lv0 = cv.take<float2>(nb);
     x.lk = cv.take<float>(w->ns ? w->ns : 1);
@@ -2265,7 +2278,7 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
   uint32_t* const rec_list = x.rec_list;
   uint32_t* const rec_n = x.rec_n;
   uint32_t* const rec_max = x.rec_max;
-  float2* const lpc = x.lpc;
+  float2* const* const lpc = x.lpc;
   float2* const la = x.la;
   float2* const lv0 = x.lv0;
   float* const lk = x.lk;
@@ -2298,44 +2311,57 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
     cudaMemcpyAsync(ss, ck + 2 * nb, slice, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(sv, ck + 3 * nb, slice, cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(rec_max, 0, sizeof(uint32_t) * S, st);
-    for (uint32_t t = 0; t < nsub; ++t) {
+    // the step kernels write the contacts and the state of every substep
+    auto record = [&](uint32_t t) {
       w->rec_list = rec_list + (size_t)REC_CAP * nb * t;
       w->rec_n = rec_n + nb * t;
       w->rec_max = rec_max + t;
-      const uint32_t sub = t % w->cfg.substeps;
-      enqueue_substep(w, dt_sub, w->old_dt, w->pending, sub == 0, sub + 1 == w->cfg.substeps);
+      w->rec_p = sp + nb * (t + 1);
+      w->rec_s = ss + nb * (t + 1);
+      w->rec_v = sv + nb * (t + 1);
+    };
+    record(0);
+    if (takes_resident(w)) {
+      e = enqueue_resident(w, dt_sub, w->old_dt, w->pending, steps);
       w->pending = false;
       if (w->any_dynamic) w->old_dt = dt_sub;
-      gather_state(w, sp + nb * (t + 1), nullptr, ss + nb * (t + 1), sv + nb * (t + 1));
+    } else {
+      for (uint32_t t = 0; t < nsub; ++t) {
+        record(t);
+        const uint32_t sub = t % w->cfg.substeps;
+        enqueue_substep(w, dt_sub, w->old_dt, w->pending, sub == 0, sub + 1 == w->cfg.substeps);
+        w->pending = false;
+        if (w->any_dynamic) w->old_dt = dt_sub;
+      }
     }
     w->rec_list = nullptr;
     w->rec_n = nullptr;
     w->rec_max = nullptr;
+    w->rec_p = w->rec_s = w->rec_v = nullptr;
+    if (e != cudaSuccess) break;
     e = cudaMemcpyAsync(hmax.data(), rec_max, sizeof(uint32_t) * nsub, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     for (uint32_t t = 0; t < nsub && e == cudaSuccess; ++t)
       if (hmax[t] > REC_CAP) status = BLOBS_ERR_OVERFLOW;  // a body with more contacts than recorded
-    // reverse substeps of the segment
-    for (int t = (int)nsub - 1; t >= 0 && status == BLOBS_OK; --t) {
+    // reverse substeps of the segment: the gather of substep t goes on to the
+    // body part of t - 1, so a segment's first launch does its body part alone
+    if (status != BLOBS_OK) break;
+    auto substep = [&](int t, int from) {
       AdjointSubstep a;
       std::memset(&a, 0, sizeof(a));
       a.p_t = sp + nb * t;
       a.s_t = ss + nb * t;
       a.v_t = w->has_springs ? sv + nb * t : nullptr;
-      a.p_t1 = sp + nb * (t + 1);
       a.s_t1 = ss + nb * (t + 1);
       a.rec_list = rec_list + (size_t)REC_CAP * nb * t;
       a.rec_n = rec_n + nb * t;
       a.spr_terms = x.spr_terms;
-      a.lp_in = adj[in][0];
-      a.lpo_in = adj[in][1];
-      a.ls_in = adj[in][2];
-      a.lv_in = adj[in][3];
-      a.lp_out = adj[in ^ 1][0];
-      a.lpo_out = adj[in ^ 1][1];
-      a.ls_out = adj[in ^ 1][2];
-      a.lv_out = adj[in ^ 1][3];
-      a.lpc = lpc;
+      a.lp_in = adj[from][0];
+      a.lpo_in = adj[from][1];
+      a.ls_in = adj[from][2];
+      a.lv_in = adj[from][3];
+      a.lpo_out = adj[from ^ 1][1];
+      a.lpc = lpc[t & 1];
       a.la = la;
       a.lv0 = lv0;
       a.lk = lk;
@@ -2343,8 +2369,17 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
       a.ratio_first = dt_sub / r.old_dt0;
       a.first_substep = (g == 0 && t == 0) ? 1u : 0u;
       a.vreq_pending = (a.first_substep && r.pending0) ? 1u : 0u;
-      launch_adjoint_substep(w->dev, a, st);
+      return a;
+    };
+    launch_adjoint_body(w->dev, substep((int)nsub - 1, in), st);
+    for (int t = (int)nsub - 1; t >= 0; --t) {
+      AdjointSubstep a = substep(t, in);
+      a.lp_out = adj[in ^ 1][0];
+      a.ls_out = adj[in ^ 1][2];
+      a.lv_out = adj[in ^ 1][3];
       in ^= 1;
+      const AdjointSubstep before = substep(t ? t - 1 : 0, in);
+      launch_adjoint_substep(w->dev, a, t ? &before : nullptr, st);
     }
   }
   w->timing = saved_timing;
