@@ -71,6 +71,7 @@ struct WorldDev {
   uint32_t* body_world;      // batched only
   uint32_t* body_col_start;  // n_bodies + 1: colliders of a body (ascending)
   uint32_t* body_cols;
+  uint32_t cols_in_order;    // body_cols[q] == q for every q
   uint32_t* body_spr_start;  // n_bodies + 1: incident springs, ascending spring index
   uint32_t* body_spr;        // (spring index << 1) | (1 if the body is endpoint b)
   uint32_t n_spr_bodies;     // single-sphere path: bodies with springs,
@@ -129,6 +130,7 @@ struct WorldDev {
   uint32_t* cell_start;      // n_cells + 1
   uint32_t* rank;            // per collider: slot inside its cell
   float4* sorted;            // per slot: (x, y, radius, collider index bits)
+  uint32_t* sorted_parent;   // per slot: the collider's body
   Contact* clist;            // general path, per collider: up to CL_CAP contacts of the substep
   uint8_t* ccount;           // general path, per collider: contacts in clist
   uint8_t* bslow;            // general path, per body: contacts need the ordered walk (zero between substeps)
@@ -270,10 +272,9 @@ __device__ __host__ __forceinline__ uint32_t cell_key(const WorldParam& wp, floa
 }
 
 // Affine2::from_angle_translation(rot, pos) * offset -> translation
-// (rigid_body.rs:88-90, physics.rs:360-366; glam Mat2 * Vec2 column form).
-__device__ __forceinline__ float2 collider_translation(float rot, float2 pos, float2 off) {
-  float s, c;
-  sincosf(rot, &s, &c);
+// (rigid_body.rs:88-90, physics.rs:360-366; glam Mat2 * Vec2 column form),
+// from the rotation's sine and cosine.
+__device__ __forceinline__ float2 collider_translation(float s, float c, float2 pos, float2 off) {
   float2 m = v2((c * off.x) + ((-s) * off.y), (s * off.x) + (c * off.y));
   return add(m, pos);
 }

@@ -1010,6 +1010,7 @@ void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const Hos
   *res_worlds = cv.take<ResWorld>(res.size());
   d.rank = cv.take<uint32_t>(nc);
   d.sorted = cv.take<float4>(sorted_storage ? 0u : nc);
+  d.sorted_parent = cv.take<uint32_t>(sorted_storage ? 0u : nc);
   d.clist = cv.take<Contact>(sorted_storage ? 0u : (size_t)nc * CL_CAP);
   d.ccount = cv.take<uint8_t>(sorted_storage ? 0u : nc);
   d.bslow = cv.take<uint8_t>(sorted_storage ? 0u : nb);
@@ -1725,6 +1726,8 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   d.n_circles = ncirc;
   d.n_cells = h.n_cells;
   d.n_tiles = n_tiles;
+  d.cols_in_order = 1u;
+  for (uint32_t q = 0; q < nc && d.cols_in_order; ++q) d.cols_in_order = h.body_cols[q] == q ? 1u : 0u;
   d.n_jblocks = h.jb_comp_start.empty() ? 0u : (uint32_t)h.jb_comp_start.size() - 1u;
   d.gravity = v2(w->cfg.gravity[0], w->cfg.gravity[1]);
   d.contacts_total = counters->contacts_total;
