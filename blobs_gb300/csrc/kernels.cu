@@ -236,6 +236,71 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(WorldDev w) {
   }
 }
 
+// Few cells: the whole scan by one block, one launch instead of two that are
+// each mostly launch and first loads (a frame of 20,000 spheres, 16,384 cells:
+// 0.48 -> 0.45 ms).  A warp takes up to SCAN_ONE_ROWS consecutive rows of 128
+// cells, all of its loads in flight.
+__global__ void __launch_bounds__(SCAN_ONE_THREADS) k_scan_one(WorldDev w) {
+  pdl_enter();
+  __shared__ uint32_t s_warp[SCAN_ONE_THREADS / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t n = w.n_cells, rows = (n + 127u) / 128u;
+  const uint32_t per = (rows + SCAN_ONE_THREADS / 32 - 1u) / (SCAN_ONE_THREADS / 32);
+  const uint32_t r0 = warp * per, r1 = min(r0 + per, rows);
+  if (threadIdx.x < COUNTER_BINS) {
+    if (w.contacts_sub) w.contacts_sub[threadIdx.x] = 0u;
+    if (w.defer_sub) w.defer_sub[threadIdx.x] = 0u;
+    if (threadIdx.x == 0 && w.defer_count) *w.defer_count = 0u;
+  }
+  uint4 v[SCAN_ONE_ROWS];
+#pragma unroll
+  for (uint32_t q = 0; q < SCAN_ONE_ROWS; ++q) {
+    const uint32_t k = (r0 + q) * 128u + lane * 4u;
+    v[q] = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + q >= r1) continue;
+    if (k + 4u <= n) {
+      v[q] = *reinterpret_cast<const uint4*>(w.cell_count + k);
+    } else {
+      if (k < n) v[q].x = w.cell_count[k];
+      if (k + 1u < n) v[q].y = w.cell_count[k + 1u];
+      if (k + 2u < n) v[q].z = w.cell_count[k + 2u];
+    }
+  }
+  uint32_t x[SCAN_ONE_ROWS], carry = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < SCAN_ONE_ROWS; ++q) {
+    const uint32_t own = (v[q].x + v[q].y) + (v[q].z + v[q].w);
+    uint32_t t = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= (uint32_t)o) t += y;
+    }
+    x[q] = carry + t - own;
+    carry += __shfl_sync(0xffffffffu, t, 31);
+  }
+  if (lane == 0) s_warp[warp] = carry;
+  __syncthreads();
+  uint32_t before = lane < warp ? s_warp[lane] : 0u;
+  before = __reduce_add_sync(0xffffffffu, before);
+#pragma unroll
+  for (uint32_t q = 0; q < SCAN_ONE_ROWS; ++q) {
+    const uint32_t k = (r0 + q) * 128u + lane * 4u;
+    if (r0 + q >= r1 || k >= n) continue;
+    const uint32_t a = before + x[q], b = a + v[q].x, c = b + v[q].y, d = c + v[q].z;
+    if (k + 4u <= n) {
+      *reinterpret_cast<uint4*>(w.cell_start + k) = make_uint4(a, b, c, d);
+      *reinterpret_cast<uint4*>(w.cell_count + k) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      w.cell_start[k] = a;
+      if (k + 1u < n) w.cell_start[k + 1u] = b;
+      if (k + 2u < n) w.cell_start[k + 2u] = c;
+      for (uint32_t i = k; i < n; ++i) w.cell_count[i] = 0u;
+    }
+    if (k + 4u >= n) w.cell_start[n] = d + v[q].w;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // gravity + springs for one body (physics.rs:369-375, springs.rs:25-47,
 // rigid_body.rs:155-160).  Springs are visited in ascending arena index and
@@ -1107,6 +1172,10 @@ void launch_keys(const WorldDev& w, bool mw, cudaStream_t st) {
 }
 
 uint32_t launch_scan(const WorldDev& w, cudaStream_t st, bool early) {
+  if (w.n_cells <= SCAN_ONE_CELLS) {
+    launch_pdl(k_scan_one, 1, SCAN_ONE_THREADS, st, early, w);
+    return 1;
+  }
   const uint32_t tiles = blocks_for(w.n_cells, SCAN_TILE);
   launch_pdl(k_tile_sums, tiles, SCAN_THREADS, st, early, w);
   if (tiles > SCAN_PREFIX_TILES && tiles == w.n_tiles) {

@@ -281,7 +281,12 @@ constexpr uint32_t DEFER_NEAR = 12;
 constexpr uint32_t WARP_NEAR = 32;
 constexpr uint32_t DEFER_CAP = 256;    // contacts a deferred body's warp ranks in shared memory
 constexpr int DEFER_THREADS = 128;
-constexpr uint32_t DEFER_BLOCKS = 152 * 8;
+// Most substeps defer no body, and the blocks started for nothing are then
+// the kernel's time: with 8 blocks per SM instead of 4 eight steps of 120k
+// spheres took 1.35 instead of 1.33 ms, four of 1M sparse ones 2.07 instead
+// of 2.04.  With 2 the ~2,900 bodies that the settled 1M pile defers wait for
+// one another (1.28 instead of 1.25 ms a step).
+constexpr uint32_t DEFER_BLOCKS = 152 * 4;
 
 template <uint32_t CAP>
 struct DeferWarp {

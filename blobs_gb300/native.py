@@ -387,8 +387,8 @@ class World:
                                                 ctypes.byref(left))
             check(st, "drain_events")
             cap = int(left.value)
-        a, b = np.zeros(max(cap, 1), np.uint32), np.zeros(max(cap, 1), np.uint32)
-        va, vb = np.zeros((max(cap, 1), 2), np.float32), np.zeros((max(cap, 1), 2), np.float32)
+        a, b = np.empty(max(cap, 1), np.uint32), np.empty(max(cap, 1), np.uint32)
+        va, vb = np.empty((max(cap, 1), 2), np.float32), np.empty((max(cap, 1), 2), np.float32)
         check(lib().blobs_world_drain_events(self._h, _ptr(a), _ptr(b), _ptr(va), _ptr(vb), cap, ctypes.byref(n),
                                              ctypes.byref(left)), "drain_events")
         k = int(n.value)

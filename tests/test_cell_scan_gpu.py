@@ -1,7 +1,8 @@
 """The cell scan (kernels.cu) at its edges, seen through SpatialHash.query:
 the queries' offsets are the scan of their counts, and query q sits on a
-cluster of q % 7 points.  Rows of 128 counts to a warp, 512 a warp, 4,096 a
-tile; more than 256 tiles take the prefix kernel."""
+cluster of q % 7 points.  One block up to 16,384 counts, in rows of 128;
+beyond, tiles of 4,096, 512 a warp; more than 256 tiles take the prefix
+kernel."""
 import numpy as np
 import pytest
 
@@ -10,8 +11,8 @@ from blobs_gb300 import native
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nq", [1, 2, 3, 4, 5, 127, 128, 129, 511, 513, 4095, 4096, 4097, 8191, 256 * 4096 - 1,
-                                256 * 4096 + 1])
+@pytest.mark.parametrize("nq", [1, 2, 3, 4, 5, 127, 128, 129, 511, 513, 4095, 4096, 4097, 8191, 16383, 16384,
+                                16385, 16386, 20_481, 256 * 4096 - 1, 256 * 4096 + 1])
 def test_offsets_of_known_counts(nq):
     centre = np.stack([np.arange(7) * 10.0, np.zeros(7)], 1).astype(np.float32)
     which = np.repeat(np.arange(7), np.arange(7))
