@@ -5,7 +5,8 @@
 //
 // Per substep, for every packed world at once:
 //   k_tile_sums,       exclusive scan of the per-cell collider counts -> cell
-//   k_scan_apply       ranges (two wait-free kernels), counts reset
+//   k_scan_apply       ranges (two wait-free kernels; k_scan_one: one for few
+//                      cells), counts reset
 //   k_scatter_forces   counting-sort scatter of the colliders into cell order
 //                      (the one-digit LSD radix pass over the cell key) and,
 //                      when springs exist, gravity + spring forces per body

@@ -12,10 +12,14 @@
 //   k_permute      (first substep of a step) storage -> this substep's cell
 //                  order; the permuted A is then also the candidate array
 //   k_scatter_cand (other substeps) a cell-order copy of A for the
-//                  candidate search (16 B per body instead of the record)
-//   k_step_single  per slot: gravity + springs, contacts over the 3x3 cells
-//                  applied in the reference's pair order, Verlet
+//                  candidate search (16 B per body instead of the record),
+//                  and the spring forces (k_springs: those alone)
+//   k_step_single  per slot: contacts over the 3x3 cells applied in the
+//                  reference's pair order, gravity and spring forces, Verlet
 //                  integration, constraints, next cell key / rank
+//   k_step_deferred  the few bodies with too many candidates, a warp each
+// or, in worlds of up to 2,048 bodies, whole steps by
+//   k_resident     a cluster of blocks per world
 // Compiled with --fmad=false (see device.cuh).
 #include "device.cuh"
 #include "kernels.h"

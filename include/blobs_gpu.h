@@ -159,7 +159,8 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt);
 /* Physics::step (physics.rs:78-82): `substeps` substeps of gravity, springs,
  * contacts, fixed joints, Verlet integration and constraints on every world. */
 int blobs_world_step(blobs_world* w, double delta);
-/* `n_steps` calls of step(delta) issued as one CUDA-graph launch. */
+/* `n_steps` calls of step(delta): launched one by one the first time this
+ * world runs that many steps of that length, one CUDA-graph launch after. */
 int blobs_world_rollout(blobs_world* w, double delta, uint32_t n_steps);
 /* Physics::fixed_step (physics.rs:84-99): accumulator with delta = 1/60 and at
  * most 3 integrate calls per frame. */
