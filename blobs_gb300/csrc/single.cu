@@ -491,7 +491,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
   const uint32_t off = incl - kk;
   for (uint32_t base = 0; base < total;) {
-    // this round: the ranges that lie wholly in [base, base + PAIR_CAP)
+    // now: the ranges that lie wholly in [base, base + PAIR_CAP)
     const bool mine = kk > 0u && off >= base && off + kk <= base + PAIR_CAP;
     const uint32_t end = __reduce_max_sync(0xffffffffu, mine ? off + kk : base);
     const uint32_t cnt = end - base, r0 = off - base;

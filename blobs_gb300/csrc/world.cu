@@ -1058,9 +1058,9 @@ bool takes_resident(const blobs_world* w) {
   return !w->res_classes.empty() && w->cfg.collisions_enabled && !w->timing && (!w->events_on || w->rec_list);
 }
 
-// `n_steps` steps of every world by the resident kernel, at most
-// RES_LAUNCH_STEPS of them to a launch.
-constexpr uint32_t RES_LAUNCH_STEPS = 64;
+// `n_steps` steps of every world by the resident kernel, as many to a launch
+// as make RES_LAUNCH_SUBSTEPS (some 10 ms).
+constexpr uint32_t RES_LAUNCH_SUBSTEPS = 1024;
 
 cudaError_t enqueue_resident(blobs_world* w, float dt, float old_dt, bool pending, uint32_t n_steps) {
   const WorldDev& d = w->dev;
@@ -1073,7 +1073,7 @@ cudaError_t enqueue_resident(blobs_world* w, float dt, float old_dt, bool pendin
   cudaError_t e = cudaSuccess;
   const size_t n_class = w->res_classes.size();
   for (uint32_t done = 0; done < n_steps && e == cudaSuccess;) {
-    const uint32_t steps = std::min(n_steps - done, RES_LAUNCH_STEPS);
+    const uint32_t steps = std::min(n_steps - done, std::max(1u, RES_LAUNCH_SUBSTEPS / w->cfg.substeps));
     e = cudaMemsetAsync(d.contacts_sub, 0, 2 * sizeof(uint32_t) * COUNTER_BINS, st);  // and defer_sub
     ResidentArgs r;
     std::memset(&r, 0, sizeof(r));

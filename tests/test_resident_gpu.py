@@ -71,7 +71,7 @@ def test_springs_static_bodies_and_crowds(n, packing, springs, statics):
     check(single(n, packing, springs=springs, statics=statics))
 
 
-@pytest.mark.parametrize("substeps,steps", [(1, 1), (1, 4), (3, 5), (7, 2), (8, 70)])
+@pytest.mark.parametrize("substeps,steps", [(1, 1), (1, 4), (3, 5), (7, 2), (8, 130), (1100, 1)])
 def test_odd_substeps_and_long_rollouts(substeps, steps):
     s = single(400, 0.6)
     s.substeps = substeps
