@@ -232,8 +232,12 @@ __device__ __forceinline__ BodyConst body_const(const WorldDev& w, const WorldPa
 
 // Exact selection walk over all candidates of the segments, in ascending
 // arena id (many candidates, or any layout): O(contacts x candidates).
-// HOOKS: the adjoint's contact recording or the event stream may be on.
-template <int MODE, bool HOOKS>
+// HOOKS: what may be on -- the adjoint's recording, the event stream (never
+// both: a recomputed substep sends no events).
+enum : int { HOOK_REC = 1, HOOK_EVENTS = 2 };
+
+
+template <int MODE, int HOOKS>
 __device__ float2 contacts_walk(const WorldDev& w, const SingleArgs& a, const Segments& g, uint32_t j, uint32_t c,
                                 float2 p0, float2 s, float r, float m, uint32_t& ncontacts, uint32_t& npush,
                                 uint32_t& nrec) {
@@ -264,11 +268,11 @@ __device__ float2 contacts_walk(const WorldDev& w, const SingleArgs& a, const Se
     single_pair(w, a, c, p0, s, r, m, best, v2(bo.x, bo.y), bo.z, m2, sp);
     if (sp.pushed) p = add(p, sp.push);
     p = add(p, sp.corr);
-    if (HOOKS && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
+    if ((HOOKS & HOOK_REC) && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
     if (best < c) {
       ++ncontacts;
       npush += sp.pushed ? 1u : 0u;
-      if (HOOKS && w.ev_rec) single_event(w, a, c, j, best);
+      if ((HOOKS & HOOK_EVENTS) && w.ev_rec) single_event(w, a, c, j, best);
     }
     last = best;
     first = false;
@@ -306,7 +310,7 @@ struct DeferWarp {
 // gravity (and the spring forces found before the contacts), Verlet, the
 // snapshot, the constraints, and the next substep's cell key and rank.  p is
 // the position after the contacts.
-template <int MODE, bool HOOKS>
+template <int MODE, int HOOKS>
 __device__ __forceinline__ void finish_single(const WorldDev& w, const SingleArgs& a, const WorldParam& wp,
                                               const BodyConst& k, uint32_t j, uint32_t c, float4 av, float4 bv,
                                               float2 p) {
@@ -360,7 +364,7 @@ __device__ __forceinline__ void finish_single(const WorldDev& w, const SingleArg
   a.a_out[j] = make_float4(snap.x, snap.y, r, av.w);
   a.b_out[j] = make_float4(p.x, p.y, po.x, po.y);
   if (a.v_vel || a.write_v) a.v_out[j] = vel;
-  if (HOOKS && a.rec_p) {  // the state after the substep for the adjoint, arena order
+  if ((HOOKS & HOOK_REC) && a.rec_p) {  // the state after the substep for the adjoint, arena order
     a.rec_p[c] = p;
     a.rec_s[c] = snap;
     if (a.v_vel) a.rec_v[c] = vel;
@@ -378,7 +382,7 @@ __device__ __forceinline__ void finish_single(const WorldDev& w, const SingleArg
 // into this thread's shared-memory slots first
 // (independent loads), then the ascending-id selection runs over shared
 // memory and only the chosen candidate's record is loaded again.
-template <int MODE, bool HOOKS, int STRIDE>
+template <int MODE, int HOOKS, int STRIDE>
 __device__ __forceinline__ float2 apply_near_s(const WorldDev& w, const SingleArgs& a, unsigned long long near,
                                                uint32_t s0, uint32_t s1, uint32_t s2, uint32_t t1, uint32_t t2,
                                                uint32_t j, uint32_t c, float2 p0, float2 s, float r, float m,
@@ -412,11 +416,11 @@ __device__ __forceinline__ float2 apply_near_s(const WorldDev& w, const SingleAr
     if (!single_pair(w, a, c, p0, s, r, m, best, v2(bo.x, bo.y), bo.z, m2, sp)) continue;
     if (sp.pushed) p = add(p, sp.push);
     p = add(p, sp.corr);
-    if (HOOKS && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
+    if ((HOOKS & HOOK_REC) && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
     if (best < c) {
       ++ncontacts;
       npush += sp.pushed ? 1u : 0u;
-      if (HOOKS && w.ev_rec) ev_lo[(nev++) * STRIDE] = best;  // appended by the warp afterwards
+      if ((HOOKS & HOOK_EVENTS) && w.ev_rec) ev_lo[(nev++) * STRIDE] = best;  // appended by the warp afterwards
     }
   }
   return p;
@@ -434,6 +438,7 @@ __device__ __forceinline__ float2 apply_near_s(const WorldDev& w, const SingleAr
 // with more than PAIR_CAP slots works in rounds of whole ranges.
 constexpr uint32_t PAIR_CAP = 128;
 
+template <bool REC>
 struct PairSlots {
   uint32_t id[PAIR_CAP];  // partner arena id
   uint32_t q[PAIR_CAP];   // partner's position in the candidate array
@@ -441,12 +446,13 @@ struct PairSlots {
   float cy[PAIR_CAP];
   uint8_t fl[PAIR_CAP];   // at the rank: 1 contact, 2 pushed out, 4 partner id below the owner's
   uint8_t own[PAIR_CAP];  // owner lane
+  uint32_t oid[REC ? PAIR_CAP : 1];  // recording: partner arena id, at the rank
 };
 
 // Correction of slot e for its owner (whose values the caller shuffled in),
 // stored at the slot's rank in the owner's range [o0, o0 + okk).
-template <int MODE>
-__device__ __forceinline__ void shared_pair(const WorldDev& w, const SingleArgs& a, PairSlots& S, uint32_t e,
+template <int MODE, bool REC>
+__device__ __forceinline__ void shared_pair(const WorldDev& w, const SingleArgs& a, PairSlots<REC>& S, uint32_t e,
                                             uint32_t jown, float2 so, float ro, float mo, uint32_t co, uint32_t o0,
                                             uint32_t okk) {
   const uint32_t id = S.id[e];
@@ -470,16 +476,17 @@ __device__ __forceinline__ void shared_pair(const WorldDev& w, const SingleArgs&
   S.cx[at] = sp.corr.x;
   S.cy[at] = sp.corr.y;
   S.fl[at] = (uint8_t)f;
+  if (REC) S.oid[at] = id;
 }
 
 // Every lane of the warp calls this; a lane with no near candidates passes
 // near = 0 and gets p back.  jbase is the slot of lane 0.
-template <int MODE>
-__device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const SingleArgs& a, PairSlots& S,
+template <int MODE, bool REC>
+__device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const SingleArgs& a, PairSlots<REC>& S,
                                                   uint32_t lane, uint32_t jbase, unsigned long long near,
                                                   uint32_t s0, uint32_t s1, uint32_t s2, uint32_t t1, uint32_t t2,
                                                   uint32_t c, float2 s, float r, float m, float2 p,
-                                                  uint32_t& ncontacts, uint32_t& npush) {
+                                                  uint32_t& ncontacts, uint32_t& npush, uint32_t& nrec) {
   const uint32_t* Cw = reinterpret_cast<const uint32_t*>(a.cand);
   const uint32_t kk = (uint32_t)__popcll(near);
   uint32_t incl = kk;
@@ -513,7 +520,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
       const float ro = __shfl_sync(0xffffffffu, r, o), mo = __shfl_sync(0xffffffffu, m, o);
       const uint32_t co = __shfl_sync(0xffffffffu, c, o);
       const uint32_t o0 = __shfl_sync(0xffffffffu, r0, o), okk = __shfl_sync(0xffffffffu, kk, o);
-      if (e < cnt) shared_pair<MODE>(w, a, S, e, jbase + o, so, ro, mo, co, o0, okk);
+      if (e < cnt) shared_pair<MODE, REC>(w, a, S, e, jbase + o, so, ro, mo, co, o0, okk);
     }
     __syncwarp();
     if (mine) {
@@ -522,6 +529,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
         if (!(f & 1u)) continue;
         if (f & 2u) p = add(p, (f & 4u) ? v2(0.01f, 0.0f) : v2(-0.01f, -0.0f));
         p = add(p, v2(S.cx[i], S.cy[i]));
+        if (REC) record_contact(w, a, c, S.oid[i], (f & 2u) != 0u, nrec);
         if (f & 4u) {
           ++ncontacts;
           npush += (f >> 1) & 1u;
@@ -642,12 +650,13 @@ __global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* 
 // consecutive slots (live: the slot holds a body).  ids, qs, ev: this
 // thread's first entries of thread-interleaved shared arrays (STRIDE threads)
 // of DEFER_NEAR entries each, pairs: the warp's.
-template <int MODE, bool HOOKS>
-__device__ constexpr bool warp_phase2() { return (MODE == 0 || MODE == 3) && !HOOKS; }
+template <int MODE, int HOOKS>
+__device__ constexpr bool warp_phase2() { return (MODE == 0 || MODE == 3) && !(HOOKS & HOOK_EVENTS); }
 
-template <int MODE, bool HOOKS, int STRIDE>
+template <int MODE, int HOOKS, int STRIDE>
 __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a, uint32_t j, bool live, uint32_t lane,
-                                          uint32_t* ids, uint32_t* qs, uint32_t* ev, PairSlots& pairs,
+                                          uint32_t* ids, uint32_t* qs, uint32_t* ev,
+                                          PairSlots<(HOOKS & HOOK_REC) != 0>& pairs,
                                           uint32_t& ncontacts, uint32_t& npush, uint32_t& nev) {
   constexpr bool WARP2 = warp_phase2<MODE, HOOKS>();
   bool deferred = false;  // contacts (and the rest of the body's substep) left to k_step_deferred
@@ -761,11 +770,11 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
           if (!single_pair(w, a, c, p0, s, r, k.m, best, v2(bo.x, bo.y), bo.z, m2, sp)) continue;
           if (sp.pushed) p = add(p, sp.push);
           p = add(p, sp.corr);
-          if (HOOKS && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
+          if ((HOOKS & HOOK_REC) && a.rec_list) record_contact(w, a, c, best, sp.pushed, nrec);
           if (best < c) {
             ++ncontacts;
             npush += sp.pushed ? 1u : 0u;
-            if (HOOKS && w.ev_rec) single_event(w, a, c, j, best);
+            if ((HOOKS & HOOK_EVENTS) && w.ev_rec) single_event(w, a, c, j, best);
           }
         }
       } else {
@@ -773,7 +782,7 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
       }
     }
     if (!WARP2 && !deferred) {
-      if (HOOKS && a.rec_list) {
+      if ((HOOKS & HOOK_REC) && a.rec_list) {
         a.rec_n[c] = nrec;
         if (nrec) atomicMax(a.rec_max, nrec);
       }
@@ -783,17 +792,23 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
   if (WARP2) {
     // (a warp without near candidates skips phase 2)
     if (a.contacts && __any_sync(0xffffffffu, wnear != 0ull))
-      p = apply_near_warp<MODE>(w, a, pairs, lane, j - lane, wnear, ws0, ws1, ws2, wt1, wt2, c,
-                                v2(av.x, av.y), av.z, k.m, p, ncontacts, npush);
+      p = apply_near_warp<MODE, (HOOKS & HOOK_REC) != 0>(w, a, pairs, lane, j - lane, wnear, ws0, ws1, ws2, wt1, wt2, c,
+                                v2(av.x, av.y), av.z, k.m, p, ncontacts, npush, nrec);
     // the records again (cache hits) rather than registers held across
     // phase 2
     if (MODE == 3 && live) wp0 = a.wparam[slot_world<MODE>(w, j)];
-    if (live && !deferred) finish_single<MODE, HOOKS>(w, a, wp0, k, j, c, a.a_in[j], a.b_in[j], p);
+    if (live && !deferred) {
+      if ((HOOKS & HOOK_REC) && a.rec_list) {
+        a.rec_n[c] = nrec;
+        if (nrec) atomicMax(a.rec_max, nrec);
+      }
+      finish_single<MODE, HOOKS>(w, a, wp0, k, j, c, a.a_in[j], a.b_in[j], p);
+    }
   }
   return deferred;
 }
 
-template <int MODE, bool HOOKS>
+template <int MODE, int HOOKS>
 __global__ void __launch_bounds__(STEP_THREADS, 8) k_step_single(WorldDev w, SingleArgs a) {
   pdl_enter();
   // phase 2 shared out over the warp (apply_near_warp): the plain step of
@@ -804,16 +819,16 @@ __global__ void __launch_bounds__(STEP_THREADS, 8) k_step_single(WorldDev w, Sin
   __shared__ uint32_t s_ids[WARP2 ? 1 : DEFER_NEAR * STEP_THREADS], s_qs[WARP2 ? 1 : DEFER_NEAR * STEP_THREADS];
   // event stream: the partners of this thread's events of phase 2, appended
   // together by the warp after it
-  __shared__ uint32_t s_ev[HOOKS ? DEFER_NEAR * STEP_THREADS : 1];
+  __shared__ uint32_t s_ev[(HOOKS & HOOK_EVENTS) ? DEFER_NEAR * STEP_THREADS : 1];
   // the near pairs of each warp
-  __shared__ PairSlots s_pairs[WARP2 ? STEP_THREADS / 32 : 1];
+  __shared__ PairSlots<(HOOKS & HOOK_REC) != 0> s_pairs[WARP2 ? STEP_THREADS / 32 : 1];
   uint32_t nev = 0, ncontacts = 0, npush = 0;
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31u;
   const bool deferred = step_slot<MODE, HOOKS, STEP_THREADS>(
       w, a, j, j < w.n_bodies, lane, s_ids + (WARP2 ? 0u : threadIdx.x), s_qs + (WARP2 ? 0u : threadIdx.x),
-      s_ev + (HOOKS ? threadIdx.x : 0u), s_pairs[WARP2 ? threadIdx.x >> 5 : 0u], ncontacts, npush, nev);
-  if (HOOKS && w.ev_rec) {
+      s_ev + ((HOOKS & HOOK_EVENTS) ? threadIdx.x : 0u), s_pairs[WARP2 ? threadIdx.x >> 5 : 0u], ncontacts, npush, nev);
+  if ((HOOKS & HOOK_EVENTS) && w.ev_rec) {
     // phase 2's events of the warp: one atomic for all of them
     uint32_t incl = nev;
 #pragma unroll
@@ -883,7 +898,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 8) k_step_single(WorldDev w, Sin
 // one lane applies them in that order -- the reference's pair order for this
 // body -- then finishes the body's substep.  More than CAP contacts:
 // the exact selection walk on one lane.
-template <int MODE, bool HOOKS, uint32_t CAP>
+template <int MODE, int HOOKS, uint32_t CAP>
 __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArgs& a, const WorldParam& wp0,
                                               DeferWarp<CAP>& S, uint32_t lane, uint32_t j, uint32_t& tc,
                                               uint32_t& tp) {
@@ -933,7 +948,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
       S.order[rank] = e;
     }
     __syncwarp();
-    if (HOOKS && w.ev_rec) {
+    if ((HOOKS & HOOK_EVENTS) && w.ev_rec) {
       // the body's events (its contacts with lower ids), appended by all
       // lanes; the host puts the buffer in the reference's order
       const uint32_t seq = *w.ev_seq;
@@ -970,13 +985,13 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
         const bool pushed = __float_as_uint(cr.z) != 0u;
         if (pushed) p = add(p, c > c2 ? v2(0.01f, 0.0f) : v2(-0.01f, -0.0f));
         p = add(p, v2(cr.x, cr.y));
-        if (HOOKS && a.rec_list) record_contact(w, a, c, c2, pushed, nrec);
+        if ((HOOKS & HOOK_REC) && a.rec_list) record_contact(w, a, c, c2, pushed, nrec);
         if (c2 < c) {
           ++tc;
           tp += pushed ? 1u : 0u;
         }
       }
-      if (HOOKS && a.rec_list) {
+      if ((HOOKS & HOOK_REC) && a.rec_list) {
         a.rec_n[c] = nrec;
         if (nrec) atomicMax(a.rec_max, nrec);
       }
@@ -987,7 +1002,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
     const float2 p = contacts_walk<MODE, HOOKS>(w, a, g, j, c, p0, s, r, k.m, nc, np, nr);
     tc += nc;
     tp += np;
-    if (HOOKS && a.rec_list) {
+    if ((HOOKS & HOOK_REC) && a.rec_list) {
       a.rec_n[c] = nr;
       if (nr) atomicMax(a.rec_max, nr);
     }
@@ -996,7 +1011,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
   __syncwarp();
 }
 
-template <int MODE, bool HOOKS>
+template <int MODE, int HOOKS>
 __global__ void __launch_bounds__(DEFER_THREADS) k_step_deferred(WorldDev w, SingleArgs a) {
   pdl_enter();
   __shared__ DeferWarp<DEFER_CAP> dsm[DEFER_THREADS / 32];
@@ -1098,17 +1113,18 @@ __device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, ui
   __syncthreads();
 }
 
+template <bool REC>
 union ResScratch {
-  PairSlots pairs[RES_WARPS];
+  PairSlots<REC> pairs[RES_WARPS];
   uint32_t ids[2][DEFER_NEAR * RES_THREADS];
   DeferWarp<RES_CAP> defer[RES_WARPS];
 };
 
-template <int MODE, bool HOOKS>  // MODE 0: uniform worlds, 1: per-body records
+template <int MODE, int HOOKS>  // MODE 0: uniform worlds, 1: per-body records
 __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentArgs r) {
   pdl_enter();
   extern __shared__ float4 s_cand[];  // the world's candidate records, then its cell table
-  __shared__ ResScratch S;
+  __shared__ ResScratch<(HOOKS & HOOK_REC) != 0> S;
   __shared__ uint32_t s_warp[RES_WARPS];
   __shared__ uint16_t s_deferred[RES_THREADS * RES_PER_THREAD];
   __shared__ uint32_t s_ndef;
@@ -1365,16 +1381,21 @@ void launch_springs(const WorldDev& w, const SingleArgs& a, cudaStream_t st) {
 void launch_step_single(const WorldDev& w, const SingleArgs& a, int mode, cudaStream_t st) {
   if (!w.n_bodies) return;
   const uint32_t g = (w.n_bodies + STEP_THREADS - 1) / STEP_THREADS;
-  if (a.rec_list || w.ev_rec) {
-    if (mode == 0) launch_pdl(k_step_single<0, true>, g, STEP_THREADS, st, true, w, a);
-    else if (mode == 1) launch_pdl(k_step_single<1, true>, g, STEP_THREADS, st, true, w, a);
-    else if (mode == 2) launch_pdl(k_step_single<2, true>, g, STEP_THREADS, st, true, w, a);
-    else launch_pdl(k_step_single<3, true>, g, STEP_THREADS, st, true, w, a);
+  if (a.rec_list) {
+    if (mode == 0) launch_pdl(k_step_single<0, HOOK_REC>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_single<1, HOOK_REC>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_single<2, HOOK_REC>, g, STEP_THREADS, st, true, w, a);
+    else launch_pdl(k_step_single<3, HOOK_REC>, g, STEP_THREADS, st, true, w, a);
+  } else if (w.ev_rec) {
+    if (mode == 0) launch_pdl(k_step_single<0, HOOK_EVENTS>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_single<1, HOOK_EVENTS>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_single<2, HOOK_EVENTS>, g, STEP_THREADS, st, true, w, a);
+    else launch_pdl(k_step_single<3, HOOK_EVENTS>, g, STEP_THREADS, st, true, w, a);
   } else {
-    if (mode == 0) launch_pdl(k_step_single<0, false>, g, STEP_THREADS, st, true, w, a);
-    else if (mode == 1) launch_pdl(k_step_single<1, false>, g, STEP_THREADS, st, true, w, a);
-    else if (mode == 2) launch_pdl(k_step_single<2, false>, g, STEP_THREADS, st, true, w, a);
-    else launch_pdl(k_step_single<3, false>, g, STEP_THREADS, st, true, w, a);
+    if (mode == 0) launch_pdl(k_step_single<0, 0>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_single<1, 0>, g, STEP_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_single<2, 0>, g, STEP_THREADS, st, true, w, a);
+    else launch_pdl(k_step_single<3, 0>, g, STEP_THREADS, st, true, w, a);
   }
 }
 
@@ -1383,24 +1404,29 @@ void launch_step_deferred(const WorldDev& w, const SingleArgs& a, int mode, cuda
   // a warp for every body at most: a 1,000-sphere world's 1,216 blocks were
   // mostly the time of starting them
   const uint32_t g = min(DEFER_BLOCKS, (w.n_bodies + DEFER_THREADS / 32 - 1) / (DEFER_THREADS / 32));
-  if (a.rec_list || w.ev_rec) {
-    if (mode == 0) launch_pdl(k_step_deferred<0, true>, g, DEFER_THREADS, st, true, w, a);
-    else if (mode == 1) launch_pdl(k_step_deferred<1, true>, g, DEFER_THREADS, st, true, w, a);
-    else if (mode == 2) launch_pdl(k_step_deferred<2, true>, g, DEFER_THREADS, st, true, w, a);
-    else launch_pdl(k_step_deferred<3, true>, g, DEFER_THREADS, st, true, w, a);
+  if (a.rec_list) {
+    if (mode == 0) launch_pdl(k_step_deferred<0, HOOK_REC>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_deferred<1, HOOK_REC>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_deferred<2, HOOK_REC>, g, DEFER_THREADS, st, true, w, a);
+    else launch_pdl(k_step_deferred<3, HOOK_REC>, g, DEFER_THREADS, st, true, w, a);
+  } else if (w.ev_rec) {
+    if (mode == 0) launch_pdl(k_step_deferred<0, HOOK_EVENTS>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_deferred<1, HOOK_EVENTS>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_deferred<2, HOOK_EVENTS>, g, DEFER_THREADS, st, true, w, a);
+    else launch_pdl(k_step_deferred<3, HOOK_EVENTS>, g, DEFER_THREADS, st, true, w, a);
   } else {
-    if (mode == 0) launch_pdl(k_step_deferred<0, false>, g, DEFER_THREADS, st, true, w, a);
-    else if (mode == 1) launch_pdl(k_step_deferred<1, false>, g, DEFER_THREADS, st, true, w, a);
-    else if (mode == 2) launch_pdl(k_step_deferred<2, false>, g, DEFER_THREADS, st, true, w, a);
-    else launch_pdl(k_step_deferred<3, false>, g, DEFER_THREADS, st, true, w, a);
+    if (mode == 0) launch_pdl(k_step_deferred<0, 0>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 1) launch_pdl(k_step_deferred<1, 0>, g, DEFER_THREADS, st, true, w, a);
+    else if (mode == 2) launch_pdl(k_step_deferred<2, 0>, g, DEFER_THREADS, st, true, w, a);
+    else launch_pdl(k_step_deferred<3, 0>, g, DEFER_THREADS, st, true, w, a);
   }
 }
 
 int launch_resident(const WorldDev& w, const ResidentArgs& r, bool uniform, uint32_t n_worlds, uint32_t shared_bytes,
                     cudaStream_t st) {
   if (!n_worlds) return 0;
-  auto kernel = r.base.rec_list ? (uniform ? k_resident<0, true> : k_resident<1, true>)
-                                : (uniform ? k_resident<0, false> : k_resident<1, false>);
+  auto kernel = r.base.rec_list ? (uniform ? k_resident<0, HOOK_REC> : k_resident<1, HOOK_REC>)
+                                : (uniform ? k_resident<0, 0> : k_resident<1, 0>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(RES_MAX_BODIES * sizeof(float4) + (RES_MAX_CELLS + 4u) * sizeof(uint32_t)));
   if (e != cudaSuccess) return (int)e;
