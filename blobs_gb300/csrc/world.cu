@@ -80,6 +80,14 @@ struct Carver {
     off = at + (bytes ? bytes : 1);
     return base ? reinterpret_cast<T*>(base + at) : nullptr;
   }
+  // where the next array starts
+  size_t mark() const { return (off + 255) & ~(size_t)255; }
+};
+
+// The part of a world's arena that a later step reads: [0, both) belongs to
+// storage buffer 0, [second, end) to buffer 1, the rest to either.
+struct StateRange {
+  size_t both = 0, second = 0, end = 0;
 };
 
 }  // namespace
@@ -213,13 +221,13 @@ struct blobs_world {
   uint32_t cur = 0;
   float2* pos[2] = {nullptr, nullptr};
   void* arena = nullptr;
-  size_t arena_bytes = 0;
-  // blobs_world_snapshot: a copy of the whole device arena (every array of
-  // the loaded scene, its cell tables and counters) and the host-side step
-  // bookkeeping that goes with it
+  StateRange state;
+  // blobs_world_snapshot: a copy of the state in the device arena
+  // ([first, first + bytes) of it) and the host-side step bookkeeping that
+  // goes with it
   struct Snapshot {
     void* mem = nullptr;
-    size_t bytes = 0;
+    size_t room = 0, first = 0, bytes = 0;
     bool valid = false;
     float old_dt = 1.0f, v_div = 0.0f;
     double time = 0.0, accumulator = 0.0;
@@ -942,28 +950,51 @@ template <class T> cudaError_t up(T* dst, const std::vector<T>& src, cudaStream_
 // Lay out (or size) every device array of the scene.
 void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const HostScene& h, uint32_t nb, uint32_t nc,
            uint32_t ns, uint32_t nj, uint32_t nw, uint32_t ncirc, uint32_t n_cells, uint32_t n_tiles,
-           bool sorted_storage, const std::vector<ResWorld>& res, ResWorld** res_worlds) {
+           bool sorted_storage, const std::vector<ResWorld>& res, ResWorld** res_worlds, StateRange& st) {
   const uint32_t ss = sorted_storage ? nb : 0u;
+  // What a later step reads comes first, so that a snapshot is one copy of
+  // it: what the one storage buffer holds, what belongs to either, what the
+  // other holds.  Everything after that is constant, or scratch that a
+  // substep writes before it reads (of a sphere world's 250 bytes a body a
+  // step reads 64 again).
   d.sa[0] = cv.take<float4>(ss);
-  d.sa[1] = cv.take<float4>(ss);
   d.sb[0] = cv.take<float4>(ss);
-  d.sb[1] = cv.take<float4>(ss);
   d.sv[0] = cv.take<float2>(ss);
-  d.sv[1] = cv.take<float2>(ss);
-  d.cand = cv.take<float4>(ss);
-  d.body_c = cv.take<float4>(ss);
+  if (!sorted_storage) pos[0] = cv.take<float2>(nb);
+  st.both = cv.mark();
   d.key = cv.take<uint32_t>(ss);
-  d.ckey = cv.take<uint32_t>(ss);
   d.where = cv.take<uint32_t>(ss);
-  d.defer_list = cv.take<uint32_t>(ss);
-  d.defer_count = cv.take<uint32_t>(sorted_storage ? 1u : 0u);
-  pos[0] = cv.take<float2>(nb);
-  pos[1] = cv.take<float2>(nb);
-  d.pos_old = cv.take<float2>(nb);
-  d.vel = cv.take<float2>(nb);
-  d.acc = cv.take<float2>(ns ? nb : 0);
+  d.rank = cv.take<uint32_t>(nc);
   d.rot = cv.take<float>(nb);
   d.angvel = cv.take<float>(nb);
+  d.cell_count = cv.take<uint32_t>(n_cells);
+  if (!sorted_storage) {
+    d.pos_old = cv.take<float2>(nb);
+    d.vel = cv.take<float2>(nb);
+    d.snap = cv.take<float2>(nc);
+    d.bslow = cv.take<uint8_t>(nb);
+  }
+  *counters = cv.take<Counters>(1);
+  st.second = cv.mark();
+  d.sa[1] = cv.take<float4>(ss);
+  d.sb[1] = cv.take<float4>(ss);
+  d.sv[1] = cv.take<float2>(ss);
+  if (!sorted_storage) pos[1] = cv.take<float2>(nb);
+  st.end = cv.mark();
+  if (sorted_storage) {  // staging of reads and writes in arena order
+    pos[0] = cv.take<float2>(nb);
+    pos[1] = cv.take<float2>(nb);
+    d.pos_old = cv.take<float2>(nb);
+    d.vel = cv.take<float2>(nb);
+    d.snap = cv.take<float2>(nc);
+    d.bslow = cv.take<uint8_t>(0);
+  }
+  d.cand = cv.take<float4>(ss);
+  d.body_c = cv.take<float4>(ss);
+  d.ckey = cv.take<uint32_t>(ss);
+  d.defer_list = cv.take<uint32_t>(ss);
+  d.defer_count = cv.take<uint32_t>(sorted_storage ? 1u : 0u);
+  d.acc = cv.take<float2>(ns ? nb : 0);
   d.mass = cv.take<float>(nb);
   d.inertia = cv.take<float>(nb);
   d.gmod = cv.take<float>(nb);
@@ -985,7 +1016,6 @@ void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const Hos
   d.col_memb = cv.take<uint32_t>(nc);
   d.col_filt = cv.take<uint32_t>(nc);
   d.col_sensor = cv.take<uint8_t>(nc);
-  d.snap = cv.take<float2>(nc);
   d.col_world = cv.take<uint32_t>(nc);
   d.spr_a = cv.take<uint32_t>(ns);
   d.spr_b = cv.take<uint32_t>(ns);
@@ -1006,20 +1036,16 @@ void carve(Carver& cv, WorldDev& d, float2** pos, Counters** counters, const Hos
   d.jb_level_start = cv.take<uint32_t>(h.jb_level_start.size());
   d.circles = cv.take<float>(3 * (size_t)ncirc);
   d.wparam = cv.take<WorldParam>(nw);
-  d.cell_count = cv.take<uint32_t>(n_cells);
   d.cell_start = cv.take<uint32_t>((size_t)n_cells + 1);
   d.cell_count_b = cv.take<uint32_t>(res.empty() ? 0u : 2 * (size_t)n_cells);
   d.key_b = cv.take<uint32_t>(res.empty() ? 0u : ss);
   d.rank_b = cv.take<uint32_t>(res.empty() ? 0u : ss);
   *res_worlds = cv.take<ResWorld>(res.size());
-  d.rank = cv.take<uint32_t>(nc);
   d.sorted = cv.take<float4>(sorted_storage ? 0u : nc);
   d.sorted_parent = cv.take<uint32_t>(sorted_storage ? 0u : nc);
   d.clist = cv.take<Contact>(sorted_storage ? 0u : (size_t)nc * CL_CAP);
   d.ccount = cv.take<uint8_t>(sorted_storage ? 0u : nc);
-  d.bslow = cv.take<uint8_t>(sorted_storage ? 0u : nb);
   d.tile_sums = cv.take<uint32_t>(n_tiles);
-  *counters = cv.take<Counters>(1);
 }
 
 }  // namespace
@@ -1706,7 +1732,6 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   w->drop_snapshot();
   if (w->arena) cudaFree(w->arena);
   w->arena = nullptr;
-  w->arena_bytes = 0;
   w->loaded = false;
 
   const uint32_t nb = scene->n_bodies, nc = scene->n_colliders, ns = scene->n_springs, nj = scene->n_joints;
@@ -1737,13 +1762,12 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   std::vector<ResWorld> res;
   w->res_classes.clear();
   if (sorted_storage && nc) resident_classes(h, *scene, nw, res, w->res_classes);
-  carve(sizer, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds);
+  carve(sizer, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds, w->state);
   e = device_alloc(w->cfg.device, &w->arena, sizer.off + 256);
   if (e != cudaSuccess) return blobs_map_cuda(e);
-  w->arena_bytes = sizer.off + 256;
   Carver cv;
   cv.base = static_cast<char*>(w->arena);
-  carve(cv, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds);
+  carve(cv, d, w->pos, &counters, h, nb, nc, ns, nj, nw, ncirc, h.n_cells, n_tiles, sorted_storage, res, &w->res_worlds, w->state);
   d.n_bodies = nb;
   d.n_cols = nc;
   d.n_springs = ns;
@@ -2043,16 +2067,22 @@ int blobs_world_snapshot(blobs_world* w) {
   if (!w->loaded) return BLOBS_ERR_STATE;
   cudaError_t e = cudaSetDevice(w->cfg.device);
   if (e != cudaSuccess) return blobs_map_cuda(e);
-  if (w->snap.bytes != w->arena_bytes) {
+  if (w->snap.room != w->state.end) {
     w->drop_snapshot();
-    e = device_alloc(w->cfg.device, &w->snap.mem, w->arena_bytes);
+    e = device_alloc(w->cfg.device, &w->snap.mem, w->state.end);
     if (e != cudaSuccess) {
       w->snap = blobs_world::Snapshot();
       return blobs_map_cuda(e);
     }
-    w->snap.bytes = w->arena_bytes;
+    w->snap.room = w->state.end;
   }
-  e = cudaMemcpyAsync(w->snap.mem, w->arena, w->arena_bytes, cudaMemcpyDeviceToDevice, w->st());
+  // the storage buffer in use, and the other too where V is kept in it (or
+  // would be without events, which may be off again by the restore)
+  const bool other = w->sorted_storage && !w->has_springs && (uint32_t)w->vbuf != w->cur;
+  w->snap.first = w->cur == 0 || other ? 0 : w->state.both;
+  w->snap.bytes = (w->cur == 1 || other ? w->state.end : w->state.second) - w->snap.first;
+  e = cudaMemcpyAsync(w->snap.mem, static_cast<char*>(w->arena) + w->snap.first, w->snap.bytes,
+                      cudaMemcpyDeviceToDevice, w->st());
   if (e != cudaSuccess) return blobs_map_cuda(e);
   w->snap.valid = true;
   w->snap.old_dt = w->old_dt;
@@ -2069,10 +2099,11 @@ int blobs_world_snapshot(blobs_world* w) {
 
 int blobs_world_restore(blobs_world* w) {
   if (!w) return BLOBS_ERR_INVALID_HANDLE;
-  if (!w->loaded || !w->snap.valid || w->snap.bytes != w->arena_bytes) return BLOBS_ERR_STATE;
+  if (!w->loaded || !w->snap.valid) return BLOBS_ERR_STATE;
   cudaError_t e = cudaSetDevice(w->cfg.device);
   if (e != cudaSuccess) return blobs_map_cuda(e);
-  e = cudaMemcpyAsync(w->arena, w->snap.mem, w->arena_bytes, cudaMemcpyDeviceToDevice, w->st());
+  e = cudaMemcpyAsync(static_cast<char*>(w->arena) + w->snap.first, w->snap.mem, w->snap.bytes,
+                      cudaMemcpyDeviceToDevice, w->st());
   if (e != cudaSuccess) return blobs_map_cuda(e);
   w->old_dt = w->snap.old_dt;
   w->v_div = w->snap.v_div;

@@ -185,11 +185,11 @@ int blobs_world_write_bodies(blobs_world* w, const float* pos, const float* pos_
 
 /* ---- snapshot / restore (no reference counterpart) -------------------------- */
 
-/* Copy the world's whole device state -- every array of the loaded scene
- * (positions, previous positions, velocities, rotations, collider snapshots,
- * pending velocity requests, cell tables, contact counters) -- and its step
- * bookkeeping (old_dt, time, fixed-step accumulator) into a snapshot the
- * world holds (one per world, device memory the size of the scene), and
+/* Copy the world's whole state -- positions, previous positions, velocities,
+ * rotations, collider snapshots, cell counts, contact counters -- and its
+ * step bookkeeping (old_dt, time, fixed-step accumulator, pending requests)
+ * into a snapshot the world holds (one per world, device memory the size of
+ * that state), and
  * restore it: stepping after a restore repeats the steps taken after the
  * snapshot bit for bit.  Device-to-device and asynchronous on the world's
  * stream.  Loading a scene drops the snapshot; restoring drops a recorded
