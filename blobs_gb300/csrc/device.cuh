@@ -366,7 +366,8 @@ constexpr int CONTACT_LIST = 24;           // per-body sorted contact list kept 
 constexpr uint32_t CL_CAP = 8;             // general path: contacts kept per collider
 constexpr uint32_t COUNTER_BINS = 64;
 constexpr uint32_t REC_CAP = 16;           // recorded contacts per body and substep (adjoint)
-constexpr int JB_THREADS = 128;            // k_joint_blocks: threads of a block, and small components at most
+constexpr uint32_t JB_COMPS = 128;         // k_joint_blocks: small components of a block at most,
+constexpr int JB_THREADS = 256;            // and its threads
 constexpr uint32_t RES_THREADS = 256;      // resident kernel: threads of a block,
 constexpr uint32_t RES_PER_THREAD = 2;     // bodies of a thread at most,
 constexpr uint32_t RES_MAX_CLUSTER = 8;    // blocks of a world at most,
@@ -374,7 +375,7 @@ constexpr uint32_t RES_MAX_BODIES = RES_THREADS * RES_PER_THREAD * RES_MAX_CLUST
 constexpr uint32_t RES_MAX_CELLS = 2 * RES_MAX_BODIES;  // and cells (what the grid cap gives that many bodies)
 constexpr uint32_t JB_MAX_JOINTS = 64;     // larger components take the coloured sweep
 constexpr uint32_t JB_JOINTS = 512;        // joints staged in shared memory per block
-constexpr uint32_t JB_BODIES = 640;        // bodies staged per block (<= JB_JOINTS + JB_THREADS)
+constexpr uint32_t JB_BODIES = 640;        // bodies staged per block (<= JB_JOINTS + JB_COMPS)
 constexpr uint32_t JB_ITERS = 4;           // iterations whose solves a block lays out in levels
 constexpr uint32_t JB_OP_BITS = 10;        // bits of a solve's joint (< JB_JOINTS), the iteration above them
 constexpr uint32_t JB_MAX_LEVELS = JB_ITERS * JB_MAX_JOINTS;  // a component's solves one after the other

@@ -507,7 +507,7 @@ int joint_schedule(uint32_t nb, uint32_t nj, const uint32_t* ja, const uint32_t*
   if (!small.empty()) {
     uint64_t tot_j = 0;
     for (uint32_t r : small) tot_j += comp_joints[r];
-    uint64_t nblk = std::max<uint64_t>({(small.size() + JB_THREADS - 1) / JB_THREADS,
+    uint64_t nblk = std::max<uint64_t>({(small.size() + JB_COMPS - 1) / JB_COMPS,
                                         (tot_j * 4 + 3 * JB_JOINTS - 1) / (3 * JB_JOINTS),
                                         ((tot_j + small.size()) * 4 + 3 * JB_BODIES - 1) / (3 * JB_BODIES), 1});
     std::vector<std::vector<uint32_t>> dealt;
@@ -521,7 +521,7 @@ int joint_schedule(uint32_t nb, uint32_t nj, const uint32_t* ja, const uint32_t*
         uint64_t k = (round & 1) ? nblk - 1 - pos : pos;
         const uint32_t cj = comp_joints[small[i]];
         uint64_t tries = 0;
-        while (dealt[k].size() == (size_t)JB_THREADS || nj_in[k] + cj > JB_JOINTS || nb_in[k] + cj + 1 > JB_BODIES) {
+        while (dealt[k].size() == (size_t)JB_COMPS || nj_in[k] + cj > JB_JOINTS || nb_in[k] + cj + 1 > JB_BODIES) {
           k = (k + 1) % nblk;
           if (++tries == nblk) {
             fits = false;
