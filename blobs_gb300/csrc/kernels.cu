@@ -334,7 +334,7 @@ __device__ __forceinline__ float2 body_forces(const WorldDev& w, uint32_t b, con
 }
 
 template <bool MW, bool SCATTER, bool SPR, bool PEND>
-__global__ void __launch_bounds__(256) k_scatter_forces(WorldDev w, const float2* __restrict__ pos) {
+__global__ void __launch_bounds__(GEN_THREADS) k_scatter_forces(WorldDev w, const float2* __restrict__ pos) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (SCATTER) {
     if (i < w.n_cols) {
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(256) k_contact_single(WorldDev w, const float2
 // left.  Loading them for every collider, and writing every collider's count
 // at its random place, four steps of that world took 3.44 ms instead of 3.24.
 template <bool MW>
-__global__ void __launch_bounds__(256) k_collider_contacts(WorldDev w, const float2* __restrict__ pos_in) {
+__global__ void __launch_bounds__(GEN_THREADS) k_collider_contacts(WorldDev w, const float2* __restrict__ pos_in) {
   const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t ncontacts = 0, npush = 0;
   if (e < w.n_cols) {
@@ -835,7 +835,7 @@ __device__ __noinline__ float2 ordered_walk(const WorldDev& w, const WorldParam&
 }
 
 template <bool MW, bool SPR, bool PEND, bool FUSE>
-__global__ void __launch_bounds__(256) k_body_contacts(WorldDev w, const float2* __restrict__ pos_in,
+__global__ void __launch_bounds__(GEN_THREADS) k_body_contacts(WorldDev w, const float2* __restrict__ pos_in,
                                                        float2* __restrict__ pos_out, SubstepArgs args) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= w.n_bodies) return;
@@ -1105,7 +1105,7 @@ __global__ void __launch_bounds__(JB_THREADS) k_joint_blocks(WorldDev w, float2*
 }
 
 template <bool MW, bool SPR, bool PEND, bool SINGLE>
-__global__ void __launch_bounds__(256) k_integrate(WorldDev w, const float2* __restrict__ pos_in,
+__global__ void __launch_bounds__(GEN_THREADS) k_integrate(WorldDev w, const float2* __restrict__ pos_in,
                                                    float2* __restrict__ pos_out, SubstepArgs args) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= w.n_bodies) return;
@@ -1204,11 +1204,11 @@ void launch_scatter_forces(const WorldDev& w, const float2* pos, bool mw, bool s
   const uint32_t nc = scatter ? w.n_cols : 0u, nb = springs ? w.n_bodies : 0u;
   const uint32_t n = nc > nb ? nc : nb;
   if (!n) return;
-  const uint32_t g = blocks_for(n, 256);
+  const uint32_t g = blocks_for(n, GEN_THREADS);
   BLOBS_DISPATCH_BOOL(mw, MW,
     BLOBS_DISPATCH_BOOL(scatter, SC,
       BLOBS_DISPATCH_BOOL(springs, SP,
-        BLOBS_DISPATCH_BOOL(pending, PE, k_scatter_forces<MW, SC, SP, PE><<<g, 256, 0, st>>>(w, pos)))));
+        BLOBS_DISPATCH_BOOL(pending, PE, k_scatter_forces<MW, SC, SP, PE><<<g, GEN_THREADS, 0, st>>>(w, pos)))));
 }
 
 uint32_t launch_contacts(const WorldDev& w, const float2* pos_in, float2* pos_out, bool mw, bool single, bool springs,
@@ -1225,14 +1225,14 @@ uint32_t launch_contacts(const WorldDev& w, const float2* pos_in, float2* pos_ou
   } else {
     if (!w.n_bodies) return 0u;
     if (w.n_cols) {
-      const uint32_t gc = blocks_for(w.n_cols, 256);
-      BLOBS_DISPATCH_BOOL(mw, MW, k_collider_contacts<MW><<<gc, 256, 0, st>>>(w, pos_in));
+      const uint32_t gc = blocks_for(w.n_cols, GEN_THREADS);
+      BLOBS_DISPATCH_BOOL(mw, MW, k_collider_contacts<MW><<<gc, GEN_THREADS, 0, st>>>(w, pos_in));
     }
-    const uint32_t g = blocks_for(w.n_bodies, 256);
+    const uint32_t g = blocks_for(w.n_bodies, GEN_THREADS);
     BLOBS_DISPATCH_BOOL(mw, MW,
       BLOBS_DISPATCH_BOOL(springs, SP,
         BLOBS_DISPATCH_BOOL(pending, PE,
-          BLOBS_DISPATCH_BOOL(fuse, FU, k_body_contacts<MW, SP, PE, FU><<<g, 256, 0, st>>>(w, pos_in, pos_out, a)))));
+          BLOBS_DISPATCH_BOOL(fuse, FU, k_body_contacts<MW, SP, PE, FU><<<g, GEN_THREADS, 0, st>>>(w, pos_in, pos_out, a)))));
     return w.n_cols ? 2u : 1u;
   }
   return 1u;
@@ -1252,11 +1252,11 @@ void launch_integrate(const WorldDev& w, const float2* pos_in, float2* pos_out, 
                       bool pending, float dt, float old_dt, bool do_keys, bool rot_dynamic, cudaStream_t st) {
   if (!w.n_bodies) return;
   SubstepArgs a{dt, old_dt, dt / old_dt, dt / dt, do_keys ? 1u : 0u, rot_dynamic ? 1u : 0u};
-  const uint32_t g = blocks_for(w.n_bodies, 256);
+  const uint32_t g = blocks_for(w.n_bodies, GEN_THREADS);
   BLOBS_DISPATCH_BOOL(mw, MW,
     BLOBS_DISPATCH_BOOL(springs, SP,
       BLOBS_DISPATCH_BOOL(pending, PE,
-        BLOBS_DISPATCH_BOOL(single, SI, k_integrate<MW, SP, PE, SI><<<g, 256, 0, st>>>(w, pos_in, pos_out, a)))));
+        BLOBS_DISPATCH_BOOL(single, SI, k_integrate<MW, SP, PE, SI><<<g, GEN_THREADS, 0, st>>>(w, pos_in, pos_out, a)))));
 }
 
 void launch_emit_pairs(const WorldDev& w, bool mw, uint32_t mode, uint32_t* out, unsigned long long cap,
