@@ -1070,10 +1070,11 @@ __device__ __forceinline__ void cluster_barrier(uint32_t n_blocks) {
   }
 }
 
-// start[k] = first + sum(count[0..k)) for k in [0, n], n a multiple of 4;
+// start[k] = first + sum(count[0..k)) for k in [0, n], n a multiple of 4, at
+// most `limit`: whatever the counts are, no range leaves the world's records;
 // every thread of the block calls it
-__device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, uint32_t first, uint32_t* start,
-                                           uint32_t* s_warp) {
+__device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, uint32_t first, uint32_t limit,
+                                           uint32_t* start, uint32_t* s_warp) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // each warp takes consecutive rows of 128 cells, four to a lane; the first
   // two rows stay in registers (all of them up to 2,048 cells)
@@ -1106,10 +1107,12 @@ __device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, ui
       if (lane >= (uint32_t)o) x += y;
     }
     const uint32_t k = r * 128u + lane * 4u, b = run + x - own;
-    if (k < n) *reinterpret_cast<uint4*>(start + k) = make_uint4(b, b + t.x, b + t.x + t.y, b + t.x + t.y + t.z);
+    if (k < n)
+      *reinterpret_cast<uint4*>(start + k) = make_uint4(min(b, limit), min(b + t.x, limit), min(b + t.x + t.y, limit),
+                                                        min(b + t.x + t.y + t.z, limit));
     run += __shfl_sync(0xffffffffu, x, 31);
   }
-  if (warp == RES_WARPS - 1u && lane == 0) start[n] = run;
+  if (warp == RES_WARPS - 1u && lane == 0) start[n] = min(run, limit);
   __syncthreads();
 }
 
@@ -1194,7 +1197,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentAr
       rq[u] = k < n ? rnk[b0 + k] : 0u;
       aq[u] = k < n ? a_cur[b0 + k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    block_scan(count + cell_base, n_cells, b0, s_start, s_warp);
+    block_scan(count + cell_base, n_cells, b0, b0 + n, s_start, s_warp);
     for (;;) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {

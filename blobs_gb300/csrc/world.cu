@@ -212,7 +212,8 @@ struct blobs_world {
   float v_div = 0.0f;           // sorted storage, V untracked: V[vbuf] holds the displacement of a substep of this dt
   int vbuf = 0;                 // sorted storage, V untracked: the V buffer in use
   bool pending = false;
-  bool keys_valid = false;
+  bool keys_valid = false;     // the keys, ranks and cell counts are those of the current snapshots
+  bool cells_counted = false;  // cell_count holds counts, whether or not they are those
   bool mass4r = false;          // sorted storage, every body's mass = 4 x radius
   std::vector<uint32_t> colour_offsets;  // colour k = joints [colour_offsets[k], colour_offsets[k+1]) in processing order
   std::vector<uint32_t> joint_order;     // processing position -> arena index
@@ -233,7 +234,7 @@ struct blobs_world {
     double time = 0.0, accumulator = 0.0;
     uint32_t cur = 0, sticky_status = 0;
     int vbuf = 0;
-    bool pending = false, keys_valid = false;
+    bool pending = false, keys_valid = false, cells_counted = false;
   } snap;
   Counters* dcounters = nullptr;
   Counters* hcounters = nullptr;  // pinned
@@ -1077,6 +1078,17 @@ void mark_end(blobs_world* w) {
   else cudaEventRecord(b, w->st());
 }
 
+// Keys, ranks and cell counts of the current snapshots, counted from zero:
+// steps without collisions move the bodies and leave the counts of the last
+// substep with them where they are.
+void recount_cells(blobs_world* w) {
+  cudaStream_t st = w->st();
+  if (w->cells_counted) cudaMemsetAsync(w->dev.cell_count, 0, sizeof(uint32_t) * (size_t)w->dev.n_cells, st);
+  if (w->sorted_storage) launch_keys_single(w->dev, w->dev.sa[w->cur], w->single_mode, st);
+  else launch_keys(w->dev, w->multiworld, st);
+  w->keys_valid = w->cells_counted = true;
+}
+
 // Does the resident kernel run this world's steps?  Not with phase
 // timing (its phases are kernels) or the event stream (ordered by substep over
 // all worlds); the reverse pass's recomputation records no events.
@@ -1092,9 +1104,8 @@ cudaError_t enqueue_resident(blobs_world* w, float dt, float old_dt, bool pendin
   const WorldDev& d = w->dev;
   cudaStream_t st = w->st();
   if (!w->keys_valid) {
-    launch_keys_single(d, d.sa[w->cur], w->single_mode, st);
+    recount_cells(w);
     w->enqueued += 1;
-    w->keys_valid = true;
   }
   cudaError_t e = cudaSuccess;
   const size_t n_class = w->res_classes.size();
@@ -1193,7 +1204,7 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     int in = cur, out = cur ^ 1;
     if (coll) {
       if (!w->keys_valid) {
-        launch_keys_single(d, d.sa[cur], w->single_mode, st);
+        recount_cells(w);
         w->enqueued += 1;
       }
       mark_begin(w, PHASE_SCAN);
@@ -1257,7 +1268,7 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     return;
   }
   if (coll && !w->keys_valid) {
-    launch_keys(d, w->multiworld, st);
+    recount_cells(w);
     w->enqueued += 1;
   }
   // Inside a graph the spring forces, which read the state at the start of
@@ -1347,11 +1358,7 @@ uint32_t f2bits(float f) {
 int launch_steady(blobs_world* w, float delta, uint32_t n_steps) {
   const float step_delta = delta / (float)w->cfg.substeps;
   const bool coll = w->cfg.collisions_enabled && w->nc > 0;
-  if (coll && !w->keys_valid) {
-    if (w->sorted_storage) launch_keys_single(w->dev, w->dev.sa[w->cur], w->single_mode, w->st());
-    else launch_keys(w->dev, w->multiworld, w->st());
-    w->keys_valid = true;
-  }
+  if (coll && !w->keys_valid) recount_cells(w);
   // the buffers baked into a graph depend on where the state is now
   GraphKey key{f2bits(delta), w->cur | ((uint32_t)w->vbuf << 1), n_steps, w->timing};
   auto it = w->graphs.find(key);
@@ -1474,7 +1481,7 @@ void restore_state(blobs_world* w, const float2* p, const float2* po, const floa
                       w->v_tracks() ? v : nullptr, sn, w->st());
   // the snapshots changed: the next substep recounts the cells from zero
   cudaMemsetAsync(w->dev.cell_count, 0, sizeof(uint32_t) * (size_t)w->dev.n_cells, w->st());
-  w->keys_valid = false;
+  w->keys_valid = w->cells_counted = false;
   w->v_div = 0.0f;
 }
 
@@ -1917,7 +1924,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   w->rot_dynamic = h.rot_dynamic;
   w->any_dynamic = h.any_dynamic;
   w->pending = h.pending;
-  w->keys_valid = false;
+  w->keys_valid = w->cells_counted = false;
   w->colour_offsets = h.colour_offsets;
   w->joint_order = h.joint_order;
   w->old_dt = old_dt;
@@ -2094,6 +2101,7 @@ int blobs_world_snapshot(blobs_world* w) {
   w->snap.vbuf = w->vbuf;
   w->snap.pending = w->pending;
   w->snap.keys_valid = w->keys_valid;
+  w->snap.cells_counted = w->cells_counted;
   return BLOBS_OK;
 }
 
@@ -2114,6 +2122,7 @@ int blobs_world_restore(blobs_world* w) {
   w->vbuf = w->snap.vbuf;
   w->pending = w->snap.pending;
   w->keys_valid = w->snap.keys_valid;
+  w->cells_counted = w->snap.cells_counted;
   w->drop_recording();  // a recorded rollout belongs to the trajectory it recorded
   return BLOBS_OK;
 }
@@ -2182,7 +2191,7 @@ int blobs_world_emit_pairs(blobs_world* w, int contacts_only, uint32_t* pairs, u
   WorldDev dv = w->dev;
   if (w->sorted_storage) {
     const int c = (int)w->cur;
-    if (!w->keys_valid) launch_keys_single(w->dev, w->dev.sa[c], w->single_mode, s);
+    if (!w->keys_valid) recount_cells(w);
     launch_scan(w->dev, s, true);
     SingleArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -2200,11 +2209,11 @@ int blobs_world_emit_pairs(blobs_world* w, int contacts_only, uint32_t* pairs, u
     if (!w->v_tracks()) w->vbuf ^= 1;
     dv.sorted = w->dev.sa[w->cur];
   } else {
-    if (!w->keys_valid) launch_keys(w->dev, w->multiworld, s);
+    if (!w->keys_valid) recount_cells(w);
     launch_scan(w->dev, s, false);
     launch_scatter_forces(w->dev, w->pos[w->cur], w->multiworld, true, false, false, s);
   }
-  w->keys_valid = false;
+  w->keys_valid = w->cells_counted = false;  // (the scan cleared the counts)
   uint32_t* dpairs = nullptr;
   unsigned long long* dcount = nullptr;
   cudaError_t e = cudaMallocAsync(&dcount, sizeof(unsigned long long), s);
