@@ -234,7 +234,7 @@ struct blobs_world {
     double time = 0.0, accumulator = 0.0;
     uint32_t cur = 0, sticky_status = 0;
     int vbuf = 0;
-    bool pending = false, keys_valid = false, cells_counted = false;
+    bool pending = false, keys_valid = false, cells_counted = false, tracked = false;
   } snap;
   Counters* dcounters = nullptr;
   Counters* hcounters = nullptr;  // pinned
@@ -1076,6 +1076,21 @@ void mark_end(blobs_world* w) {
   cudaEvent_t b = w->recording->marks.back().b;
   if (w->capturing) cudaEventRecordWithFlags(b, w->st(), cudaEventRecordExternal);
   else cudaEventRecord(b, w->st());
+}
+
+// V after a change of v_tracks(): from the buffer of its own, a displacement
+// perhaps, to calculated_velocity double-buffered with the state, or back.
+cudaError_t retrack_v(blobs_world* w) {
+  const int c = (int)w->cur;
+  cudaError_t e = cudaSuccess;
+  if (w->v_tracks()) {
+    if (w->vbuf != c) e = cudaMemcpyAsync(w->dev.sv[c], w->dev.sv[w->vbuf], sizeof(float2) * w->nb,
+                                          cudaMemcpyDeviceToDevice, w->st());
+    if (e == cudaSuccess && w->v_div != 0.0f) launch_v_divide(w->dev.sv[c], w->nb, w->v_div, w->st());
+  }
+  w->vbuf = c;
+  w->v_div = 0.0f;
+  return e;
 }
 
 // Keys, ranks and cell counts of the current snapshots, counted from zero:
@@ -2083,9 +2098,8 @@ int blobs_world_snapshot(blobs_world* w) {
     }
     w->snap.room = w->state.end;
   }
-  // the storage buffer in use, and the other too where V is kept in it (or
-  // would be without events, which may be off again by the restore)
-  const bool other = w->sorted_storage && !w->has_springs && (uint32_t)w->vbuf != w->cur;
+  // the storage buffer in use, and the other too where V is kept in it
+  const bool other = w->sorted_storage && !w->v_tracks() && (uint32_t)w->vbuf != w->cur;
   w->snap.first = w->cur == 0 || other ? 0 : w->state.both;
   w->snap.bytes = (w->cur == 1 || other ? w->state.end : w->state.second) - w->snap.first;
   e = cudaMemcpyAsync(w->snap.mem, static_cast<char*>(w->arena) + w->snap.first, w->snap.bytes,
@@ -2102,6 +2116,7 @@ int blobs_world_snapshot(blobs_world* w) {
   w->snap.pending = w->pending;
   w->snap.keys_valid = w->keys_valid;
   w->snap.cells_counted = w->cells_counted;
+  w->snap.tracked = w->v_tracks();
   return BLOBS_OK;
 }
 
@@ -2124,7 +2139,9 @@ int blobs_world_restore(blobs_world* w) {
   w->keys_valid = w->snap.keys_valid;
   w->cells_counted = w->snap.cells_counted;
   w->drop_recording();  // a recorded rollout belongs to the trajectory it recorded
-  return BLOBS_OK;
+  // the event stream was switched on or off in between
+  if (w->sorted_storage && w->v_tracks() != w->snap.tracked) e = retrack_v(w);
+  return blobs_map_cuda(e);
 }
 
 int blobs_world_joint_order(blobs_world* w, uint32_t* order, uint32_t* n_colours) {
@@ -2516,17 +2533,7 @@ int blobs_world_set_events(blobs_world* w, int enabled, uint32_t capacity) {
     if (e != cudaSuccess) return blobs_map_cuda(e);
     w->events_on = true;
   }
-  if (w->loaded && w->sorted_storage && !w->has_springs && w->events_on != was_on) {
-    const int c = (int)w->cur;
-    if (w->events_on) {
-      // V becomes calculated_velocity, double-buffered with the state
-      if (w->vbuf != c) e = cudaMemcpyAsync(w->dev.sv[c], w->dev.sv[w->vbuf], sizeof(float2) * w->nb,
-                                            cudaMemcpyDeviceToDevice, st);
-      if (e == cudaSuccess && w->v_div != 0.0f) launch_v_divide(w->dev.sv[c], w->nb, w->v_div, st);
-    }
-    w->vbuf = c;
-    w->v_div = 0.0f;
-  }
+  if (w->loaded && w->sorted_storage && !w->has_springs && w->events_on != was_on) e = retrack_v(w);
   w->attach_events();
   if (e == cudaSuccess) e = cudaGetLastError();
   return blobs_map_cuda(e);
