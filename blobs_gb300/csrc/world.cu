@@ -1483,21 +1483,21 @@ int run_steps(blobs_world* w, double delta, uint32_t n_steps) {
 }
 
 // Arena-order state (p, po, s, v) of a single-sphere world into four
-// n-body float2 slices (v only holds velocities in worlds with springs).
+// n-body float2 slices, v as calculated_velocity.
 void gather_state(blobs_world* w, float2* p, float2* po, float2* sn, float2* v) {
   const int c = (int)w->cur;
   launch_gather_single(w->dev, w->dev.sa[c], w->dev.sb[c], w->dev.sv[w->v_tracks() ? c : w->vbuf], p, po,
-                       w->v_tracks() ? v : nullptr, sn, 0.0f, w->st());
+                       v, sn, w->v_div, w->st());
 }
 
 void restore_state(blobs_world* w, const float2* p, const float2* po, const float2* sn, const float2* v) {
   const int c = (int)w->cur;
   launch_write_single(w->dev, w->dev.sa[c], w->dev.sb[c], w->dev.sv[w->v_tracks() ? c : w->vbuf], p, po,
-                      w->v_tracks() ? v : nullptr, sn, w->st());
+                      v, sn, w->st());
   // the snapshots changed: the next substep recounts the cells from zero
   cudaMemsetAsync(w->dev.cell_count, 0, sizeof(uint32_t) * (size_t)w->dev.n_cells, w->st());
   w->keys_valid = w->cells_counted = false;
-  w->v_div = 0.0f;
+  w->v_div = 0.0f;  // every V entry is now a velocity
 }
 
 int read_status(blobs_world* w) {
@@ -2286,8 +2286,6 @@ int blobs_world_rollout_record(blobs_world* w, double delta, uint32_t n_steps, u
   const size_t nb = w->nb;
   cudaError_t e = pool_alloc(w->cfg.device, &r.ckpt, sizeof(float2) * 4 * nb * (n_seg + 1), w->st());
   if (e != cudaSuccess) return blobs_map_cuda(e);
-  // v is only gathered in worlds that track it
-  if (!w->v_tracks()) e = cudaMemsetAsync(r.ckpt, 0, sizeof(float2) * 4 * nb * (n_seg + 1), w->st());
   r.delta = delta;
   r.n_steps = n_steps;
   r.every = checkpoint_every;

@@ -1,0 +1,49 @@
+"""The reverse pass leaves the world in the rollout's final state, velocities
+included: reads before and after it are equal and so are the steps that
+follow, in worlds that keep velocities in another form while nothing reads
+them during a step (no springs, no events) as in those that do not."""
+import numpy as np
+import pytest
+
+from blobs_gb300 import native, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def world(n, springs):
+    s = scenes.random_world(np.random.Generator(np.random.PCG64(n)), n, 0.1, 0.2, 0.3, 1.0, spring_frac=springs)
+    s.dt = 1.0 / 60.0
+    return s
+
+
+WORLDS = {
+    "resident": lambda springs: world(700, springs),
+    "spheres": lambda springs: world(5000, springs),
+    "batch": lambda springs: scenes.pack([world(200 + k, springs) for k in range(12)]),
+}
+
+
+def state(w):
+    b = w.read_bodies()
+    return [b[k] for k in ("pos", "pos_old", "vel", "rotation", "angvel")] + [w.read_snapshots()]
+
+
+@pytest.mark.parametrize("events", [False, True])
+@pytest.mark.parametrize("springs", [0.0, 0.3])
+@pytest.mark.parametrize("steps,every", [(1, 1), (3, 2), (4, 2)])
+@pytest.mark.parametrize("name", list(WORLDS))
+def test_reverse_pass_leaves_the_velocities(name, springs, steps, every, events):
+    s = WORLDS[name](springs)
+    g = np.linspace(-1.0, 1.0, 2 * s.n_bodies, dtype=np.float32).reshape(-1, 2)
+    with native.World(s) as w, native.World(s) as plain:
+        if events:
+            w.set_events(True, 1 << 20)
+        w.rollout_record(s.dt, steps, every)
+        plain.rollout(s.dt, steps)
+        want = state(w)
+        assert all(np.array_equal(a, b) for a, b in zip(want, state(plain)))
+        w.backward(g, s.n_springs)
+        assert all(np.array_equal(a, b) for a, b in zip(state(w), want))
+        w.step(s.dt)
+        plain.step(s.dt)
+        assert all(np.array_equal(a, b) for a, b in zip(state(w), state(plain)))
