@@ -2330,6 +2330,7 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
     float4* spr_terms;
     float* lk;
     Counters* saved;
+    float *rot, *angvel;
   } x;
   auto lay = [&](Carver& cv) {
     x.sp = cv.take<float2>(nb * (S + 1));  // p, s, v of every recorded state
@@ -2346,6 +2347,8 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
     x.lv0 = cv.take<float2>(nb);
     x.lk = cv.take<float>(w->ns ? w->ns : 1);
     x.saved = cv.take<Counters>(1);
+    x.rot = cv.take<float>(w->rot_dynamic ? nb : 0);
+    x.angvel = cv.take<float>(w->rot_dynamic ? nb : 0);
   };
   Carver sizer;
   lay(sizer);
@@ -2374,6 +2377,9 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
   if (e == cudaSuccess) e = cudaMemsetAsync(lv0, 0, slice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(lk, 0, sizeof(float) * (w->ns ? w->ns : 1), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(saved, w->dcounters, sizeof(Counters), cudaMemcpyDeviceToDevice, st);
+  // the recomputed substeps turn the bodies once more, which nothing else reads
+  if (e == cudaSuccess && w->rot_dynamic) e = cudaMemcpyAsync(x.rot, w->dev.rot, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess && w->rot_dynamic) e = cudaMemcpyAsync(x.angvel, w->dev.angvel, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st);
   int in = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(adj[in][0], dl_dpos, slice, cudaMemcpyHostToDevice, st);
   const float dt_sub = (float)r.delta / (float)w->cfg.substeps;
@@ -2483,6 +2489,8 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
     w->old_dt = dt_sub;
     w->pending = false;
     e = cudaMemcpyAsync(w->dcounters, saved, sizeof(Counters), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && w->rot_dynamic) e = cudaMemcpyAsync(w->dev.rot, x.rot, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && w->rot_dynamic) e = cudaMemcpyAsync(w->dev.angvel, x.angvel, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st);
   }
   cudaFreeAsync(buf, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
