@@ -1450,6 +1450,14 @@ int launch_steady(blobs_world* w, float delta, uint32_t n_steps) {
   return BLOBS_OK;
 }
 
+// Is the caller capturing the world's stream into a graph of their own?  What
+// is queued then runs when and as often as that graph is launched, but the
+// storage buffers of steps alternate and the host keeps track of them.
+bool under_capture(const blobs_world* w) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return w->user_stream && (cudaStreamIsCapturing(w->user_stream, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone);
+}
+
 int run_steps(blobs_world* w, double delta, uint32_t n_steps) {
   if (!w->loaded) return BLOBS_ERR_STATE;
   if (!(delta > 0.0) || !std::isfinite(delta)) return BLOBS_ERR_INVALID_ARGUMENT;
@@ -1458,8 +1466,10 @@ int run_steps(blobs_world* w, double delta, uint32_t n_steps) {
   const float df = (float)delta;
   const float step_delta = df / (float)w->cfg.substeps;
   uint32_t done = 0;
+  auto irregular = [&] { return w->pending || (w->any_dynamic && f2bits(w->old_dt) != f2bits(step_delta)); };
+  if (n_steps > (irregular() ? 1u : 0u) && under_capture(w)) return BLOBS_ERR_CUDA;
   // irregular first step: eager
-  while (done < n_steps && (w->pending || (w->any_dynamic && f2bits(w->old_dt) != f2bits(step_delta)))) {
+  while (done < n_steps && irregular()) {
     if (w->timing) {
       w->recording = &w->eager_timing;
       if (std::find(w->launched_sets.begin(), w->launched_sets.end(), w->recording) == w->launched_sets.end())
@@ -1967,12 +1977,15 @@ int blobs_world_fixed_step(blobs_world* w, double frame_time) {
   if (!w) return BLOBS_ERR_INVALID_HANDLE;
   if (!w->loaded) return BLOBS_ERR_STATE;
   // physics.rs:84-99
+  const double delta = 1.0 / 60.0, before = w->accumulator;
   w->accumulator += frame_time;
-  const double delta = 1.0 / 60.0;
   int max_steps = 3;
   while (w->accumulator >= delta && max_steps > 0) {
     int st = run_steps(w, delta, 1);
-    if (st) return st;
+    if (st) {
+      if (max_steps == 3) w->accumulator = before;  // nothing ran
+      return st;
+    }
     w->accumulator -= delta;
     max_steps -= 1;
   }
@@ -2280,6 +2293,7 @@ int blobs_world_rollout_record(blobs_world* w, double delta, uint32_t n_steps, u
   if (!w->loaded) return BLOBS_ERR_STATE;
   if (!w->sorted_storage || w->ncirc || n_steps == 0 || checkpoint_every == 0) return BLOBS_ERR_INVALID_ARGUMENT;
   cudaSetDevice(w->cfg.device);
+  if (under_capture(w)) return BLOBS_ERR_CUDA;
   auto& r = w->rec;
   w->drop_recording();
   const uint32_t n_seg = (n_steps + checkpoint_every - 1) / checkpoint_every;
@@ -2316,6 +2330,7 @@ int blobs_world_backward(blobs_world* w, const float* dl_dpos, float* dl_dvreq, 
   if (!w->loaded || !w->rec.valid || w->rec.substeps != w->cfg.substeps) return BLOBS_ERR_STATE;
   if (!dl_dpos) return BLOBS_ERR_INVALID_ARGUMENT;
   cudaSetDevice(w->cfg.device);
+  if (under_capture(w)) return BLOBS_ERR_CUDA;
   auto& r = w->rec;
   const size_t nb = w->nb;
   const uint32_t S = r.every * w->cfg.substeps;  // substeps per full segment

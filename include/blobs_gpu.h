@@ -170,7 +170,13 @@ int blobs_world_sync(blobs_world* w);
 
 /* Run the world's work on the caller's CUDA stream (a cudaStream_t) instead of
  * its own; NULL returns to the world's own stream.  Lets a host order the
- * step with its own copies and kernels. */
+ * step with its own copies and kernels.  While the caller captures that stream
+ * into a graph of their own, steps and rollouts are refused with
+ * BLOBS_ERR_CUDA, nothing queued and nothing changed: a step's storage buffers
+ * alternate with the host's bookkeeping, which a replay would leave behind.
+ * (The one exception is a single first step, or first step of another length:
+ * it is queued, and right if that graph is launched once before any other
+ * call.) */
 int blobs_world_set_stream(blobs_world* w, void* stream);
 
 /* ---- host writes between steps ----------------------------------------------- */
