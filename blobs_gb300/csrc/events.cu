@@ -26,8 +26,8 @@ __device__ __forceinline__ uint32_t event_bucket(const EventSort& s, uint4 r) {
 }
 
 // first event of each substep of the batch: off[k] = lower bound of seq0 + k
-__global__ void __launch_bounds__(256) k_ev_bounds(const uint4* __restrict__ rec, uint32_t n, uint32_t seq0,
-                                                   uint32_t n_seq, uint32_t stride, uint32_t* __restrict__ off,
+__global__ void __launch_bounds__(256) k_ev_bounds(const uint4* rec, uint32_t n, uint32_t seq0,
+                                                   uint32_t n_seq, uint32_t stride, uint32_t* off,
                                                    uint32_t n_off) {
   pdl_enter();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -604,8 +604,8 @@ __device__ __forceinline__ void spring_slot(const WorldDev& w, const SingleArgs&
   if (c < w.n_bodies && ((w.spr_bits[c >> 5] >> (c & 31u)) & 1u)) spring_body(w, a.b_in, a.v_in, a.pending, c);
 }
 
-__global__ void __launch_bounds__(256) k_springs(WorldDev w, const float4* __restrict__ b_in,
-                                                 const float2* __restrict__ v_in, uint32_t pending) {
+__global__ void __launch_bounds__(256) k_springs(WorldDev w, const float4* b_in,
+                                                 const float2* v_in, uint32_t pending) {
   pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < w.n_spr_bodies) spring_body(w, b_in, v_in, pending, w.spr_bodies[i]);
@@ -618,10 +618,10 @@ __global__ void __launch_bounds__(256) k_springs(WorldDev w, const float4* __res
 // springs: a batch of 1,024 worlds with springs on a fifth of the bodies took
 // 5.69 ms for four steps instead of 5.55 (with springs on 63% of them, as in
 // the 256 x 2,048 batch, the two are within 2%).
-__global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* __restrict__ a_in,
-                                                      float4* __restrict__ cand, uint32_t copy_blocks,
-                                                      const float4* __restrict__ b_in,
-                                                      const float2* __restrict__ v_in, uint32_t pending) {
+__global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* a_in,
+                                                      float4* cand, uint32_t copy_blocks,
+                                                      const float4* b_in,
+                                                      const float2* v_in, uint32_t pending) {
   pdl_enter();
   if (blockIdx.x >= copy_blocks) {
     const uint32_t i = (blockIdx.x - copy_blocks) * blockDim.x + threadIdx.x;
@@ -1293,7 +1293,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentAr
 }
 
 // Keys and ranks of the current storage (after a load or a host write).
-__global__ void __launch_bounds__(256) k_keys_single(WorldDev w, const float4* __restrict__ A, int mode) {
+__global__ void __launch_bounds__(256) k_keys_single(WorldDev w, const float4* A, int mode) {
   pdl_enter();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= w.n_bodies) return;
@@ -1307,8 +1307,8 @@ __global__ void __launch_bounds__(256) k_keys_single(WorldDev w, const float4* _
 }
 
 // Storage order -> arena order (reads) and back (host writes).
-__global__ void __launch_bounds__(256) k_gather_single(WorldDev w, const float4* __restrict__ A,
-                                                       const float4* __restrict__ B, const float2* __restrict__ V,
+__global__ void __launch_bounds__(256) k_gather_single(WorldDev w, const float4* A,
+                                                       const float4* B, const float2* V,
                                                        float2* pos, float2* pos_old, float2* vel, float2* snap,
                                                        float v_div) {
   pdl_enter();

@@ -115,8 +115,8 @@ constexpr uint32_t SH_RANKED = 64;  // results up to this many are ranked agains
 // WRITE = false: count the matches into qcount; WRITE = true: the matches'
 // ids ascending from qstart[q] on in `out` (`tmp`: as much scratch, or NULL).
 template <bool WRITE>
-__global__ void __launch_bounds__(256) k_sh_query(HashDev h, uint32_t nq, const float2* __restrict__ qxy,
-                                                  const float* __restrict__ qr, uint32_t* qcount,
+__global__ void __launch_bounds__(256) k_sh_query(HashDev h, uint32_t nq, const float2* qxy,
+                                                  const float* qr, uint32_t* qcount,
                                                   const uint32_t* qstart, unsigned long long* tmp,
                                                   unsigned long long* out, unsigned long long cap) {
   pdl_enter();
@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(256) k_sh_query(HashDev h, uint32_t nq, const 
 
 // The queries' starts as the 64-bit offsets that are handed out; the flag: a
 // prefix wrapped (more than 2^32 - 1 results).
-__global__ void __launch_bounds__(256) k_sh_offsets(const uint32_t* __restrict__ start, uint32_t n,
-                                                    unsigned long long* __restrict__ offsets) {
+__global__ void __launch_bounds__(256) k_sh_offsets(const uint32_t* start, uint32_t n,
+                                                    unsigned long long* offsets) {
   pdl_enter();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
