@@ -168,16 +168,36 @@ struct WorldDev {
 
 // First statement, before any read of memory, of the kernels that launch_pdl
 // (kernels.h) starts: waits until the kernels before it are complete and
-// their writes visible, then lets the next kernel in the stream be placed on
-// the SMs once all blocks of this one have come this far.  A single-sphere
+// their writes visible (pdl_wait), then lets the next kernel in the stream be
+// placed on the SMs once all blocks of this one have come this far.  A single-sphere
 // substep is five dependent kernels, a few microseconds each in small
 // worlds; the launch of one hides behind the run of the one before it (1M
 // sparse spheres: 2.28 -> 2.19 ms for four steps; the eager launches of a
 // small gradient: 1.76 -> 1.33 ms).  The trigger stands after the wait:
 // before it, whole chains of waiting kernels filled the SMs.
+//
+// A kernel in front of k_step_single, and the step's blocks all on the SMs at
+// once (up to PDL_LATE_BODIES): the wait alone, and the step is placed when
+// all blocks of this one are done.  Placed earlier, into what the running
+// blocks left free, its blocks were spread unevenly over the SMs, and the
+// fullest SM decided.  Settled piles, us a step, plain launches / early / at
+// the end: 30k bodies 330 / 360 / 306, 60k 416 / 443 / 389, 100k 503 / 544 /
+// 477, 60k over twice their box's area 812 / 955 / 797; 20k sparse 124 / 102 /
+// 99.  Several waves even themselves out (four steps of 1M spheres 2.35 early,
+// 2.37 ms at the end).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+constexpr int STEP_THREADS = 128;     // k_step_single, eight blocks to an SM
+constexpr uint32_t PDL_LATE_BODIES = 152 * 8 * STEP_THREADS;
+
+__device__ __forceinline__ void pdl_enter_before_step(uint32_t n_bodies) {
+  pdl_wait();
+  if (n_bodies > PDL_LATE_BODIES) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

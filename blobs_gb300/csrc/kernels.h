@@ -5,8 +5,9 @@
 
 namespace blobs {
 
-// Launches a kernel that begins with pdl_enter() (device.cuh); early: its
-// blocks may take their places while the kernel before it still drains.  The
+// Launches a kernel that begins with pdl_enter() or pdl_enter_before_step()
+// (device.cuh); early: its blocks may take their places while the kernel
+// before it still drains.  The
 // general path's chain of kernels is launched without: there the waiting
 // blocks cost more than the launches (200k jointed bodies, four steps: 4.64
 // ms with, 3.64 ms without).  Such a kernel starts while the one before it

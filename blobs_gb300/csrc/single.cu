@@ -280,8 +280,6 @@ __device__ float2 contacts_walk(const WorldDev& w, const SingleArgs& a, const Se
   return p;
 }
 
-constexpr int STEP_THREADS = 128;
-
 // Bodies with more near candidates than this take k_step_deferred (the
 // per-lane ordered selection is O(near^2)); with phase 2 shared out over
 // the warp, more than WARP_NEAR.
@@ -544,7 +542,7 @@ __device__ __forceinline__ float2 apply_near_warp(const WorldDev& w, const Singl
 
 // Storage slot i -> its position in this substep's cell order.
 __global__ void __launch_bounds__(256) k_permute(WorldDev w, SingleArgs a) {
-  pdl_enter();
+  pdl_enter_before_step(w.n_bodies);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= w.n_bodies) return;
   const uint32_t key = w.key[i];
@@ -606,7 +604,7 @@ __device__ __forceinline__ void spring_slot(const WorldDev& w, const SingleArgs&
 
 __global__ void __launch_bounds__(256) k_springs(WorldDev w, const float4* b_in,
                                                  const float2* v_in, uint32_t pending) {
-  pdl_enter();
+  pdl_enter_before_step(w.n_bodies);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < w.n_spr_bodies) spring_body(w, b_in, v_in, pending, w.spr_bodies[i]);
 }
@@ -622,7 +620,7 @@ __global__ void __launch_bounds__(256) k_scatter_cand(WorldDev w, const float4* 
                                                       float4* cand, uint32_t copy_blocks,
                                                       const float4* b_in,
                                                       const float2* v_in, uint32_t pending) {
-  pdl_enter();
+  pdl_enter_before_step(w.n_bodies);
   if (blockIdx.x >= copy_blocks) {
     const uint32_t i = (blockIdx.x - copy_blocks) * blockDim.x + threadIdx.x;
     if (i < w.n_spr_bodies) spring_body(w, b_in, v_in, pending, w.spr_bodies[i]);

@@ -27,7 +27,7 @@ def test_kernels_launched_early_wait_first_and_read_coherently():
     for _, text in sources():
         launched |= set(re.findall(r"launch_pdl\((k_\w+)", text))
         for name, params, first in kernels(text):
-            if re.match(r"\s*pdl_\w+\(\)\s*;", first):
+            if re.match(r"\s*pdl_\w+\([\w.]*\)\s*;", first):
                 waiting[name] = params
     assert len(launched) > 15
     assert launched <= set(waiting), sorted(launched - set(waiting))
