@@ -177,14 +177,15 @@ struct WorldDev {
 // before it, whole chains of waiting kernels filled the SMs.
 //
 // A kernel in front of k_step_single, and the step's blocks all on the SMs at
-// once (up to PDL_LATE_BODIES): the wait alone, and the step is placed when
-// all blocks of this one are done.  Placed earlier, into what the running
-// blocks left free, its blocks were spread unevenly over the SMs, and the
-// fullest SM decided.  Settled piles, us a step, plain launches / early / at
-// the end: 30k bodies 330 / 360 / 306, 60k 416 / 443 / 389, 100k 503 / 544 /
+// once, more than one to an SM (pdl_late): the wait alone, and the step is
+// placed when all blocks of this one are done.  Placed earlier, into what the
+// running blocks left free, its blocks were spread unevenly over the SMs, and
+// the fullest SM decided.  Settled piles, us a step, plain launches / early /
+// at the end: 30k bodies 330 / 360 / 306, 60k 416 / 443 / 389, 100k 503 / 544 /
 // 477, 60k over twice their box's area 812 / 955 / 797; 20k sparse 124 / 102 /
 // 99.  Several waves even themselves out (four steps of 1M spheres 2.35 early,
-// 2.37 ms at the end).
+// 2.37 ms at the end), and with a block to an SM there is no choice (eight
+// steps of 10.6k sparse spheres 0.794 early, 0.806 ms at the end).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void pdl_enter() {
@@ -193,11 +194,13 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 constexpr int STEP_THREADS = 128;     // k_step_single, eight blocks to an SM
-constexpr uint32_t PDL_LATE_BODIES = 152 * 8 * STEP_THREADS;
+__device__ __forceinline__ bool pdl_late(uint32_t n_bodies) {
+  return n_bodies > 152 * STEP_THREADS && n_bodies <= 152 * 8 * STEP_THREADS;
+}
 
 __device__ __forceinline__ void pdl_enter_before_step(uint32_t n_bodies) {
   pdl_wait();
-  if (n_bodies > PDL_LATE_BODIES) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!pdl_late(n_bodies)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

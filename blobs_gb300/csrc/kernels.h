@@ -7,13 +7,12 @@ namespace blobs {
 
 // Launches a kernel that begins with pdl_enter() or pdl_enter_before_step()
 // (device.cuh); early: its blocks may take their places while the kernel
-// before it still drains.  The
-// general path's chain of kernels is launched without: there the waiting
-// blocks cost more than the launches (200k jointed bodies, four steps: 4.64
-// ms with, 3.64 ms without).  Such a kernel starts while the one before it
-// still writes what it is going to read, so none of its pointers is
-// __restrict__: that would let the compiler read through the non-coherent
-// path, or move a load up across the wait.
+// before it still drains.  The general path's chain of kernels is launched
+// without: there the waiting blocks cost more than the launches (200k jointed
+// bodies, four steps: 4.64 ms with, 3.64 ms without).  Such a kernel starts
+// while the one before it still writes what it is going to read, so none of
+// its pointers is __restrict__: that would let the compiler read through the
+// non-coherent path, or move a load up across the wait.
 template <class... P, class... A>
 inline void launch_pdl(void (*k)(P...), uint32_t grid, uint32_t threads, cudaStream_t st, bool early, A&&... a) {
   cudaLaunchConfig_t cfg{};
