@@ -445,7 +445,15 @@ __device__ __forceinline__ void integrate_body(const WorldDev& w, uint32_t b, fl
 // contiguous range of the cell-sorted array (split in two where the torus
 // wraps).
 // ---------------------------------------------------------------------------
-template <class F>
+//
+// FLAT: the three rows as one sequence, their six bounds loaded together, so
+// that a warp runs as long as its longest sum of rows, not the sum of its
+// longest rows (k_collider_contacts, 200k bodies, four steps: 3.24 -> 3.17 ms;
+// records loaded two or four at a time were slower, 3.31 and 3.27).  The walks
+// over crowded bodies are long rows, and pay for the choice of row at each
+// candidate (50k bodies at 16 times that density: 11.9 ms a step by rows,
+// 12.7 flat).
+template <bool FLAT = false, class F>
 __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const WorldParam& wp, float2 s, F&& f) {
   const uint32_t wm = (1u << wp.log2w) - 1u, hm = (1u << wp.log2h) - 1u;
   const uint32_t ix = (uint32_t)grid_coord(s.x, wp.ox, wp.inv_cs), iy = (uint32_t)grid_coord(s.y, wp.oy, wp.inv_cs);
@@ -453,7 +461,7 @@ __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const Worl
   const uint32_t n = w.n_cols;
   // ranges are clamped to the slot count: a corrupt cell table cannot walk
   // past the sorted array
-  if (x0 < x2) {
+  if (FLAT && x0 < x2) {
     uint32_t b[3], e[3];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
@@ -461,10 +469,6 @@ __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const Worl
       b[r] = w.cell_start[row + x0];
       e[r] = w.cell_start[row + x2 + 1u];
     }
-    // The three rows as one sequence: their six bounds are loaded together,
-    // and a warp runs as long as its longest sum of rows, not the sum of its
-    // longest rows (200k bodies, four steps: 3.24 -> 3.17 ms).  Records loaded
-    // two or four at a time were slower (3.31, 3.27).
     const uint32_t l0 = min(e[0], n) > b[0] ? min(e[0], n) - b[0] : 0u, l1 = min(e[1], n) > b[1] ? min(e[1], n) - b[1] : 0u,
                    l2 = min(e[2], n) > b[2] ? min(e[2], n) - b[2] : 0u;
     const uint32_t m = l0 + l1 + l2;
@@ -474,10 +478,15 @@ __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const Worl
 #pragma unroll 1
   for (int oy = -1; oy <= 1; ++oy) {
     const uint32_t row = wp.cell_base + (((iy + (uint32_t)oy) & hm) << wp.log2w);
-    uint32_t e0 = w.cell_start[row + x0], e1 = min(w.cell_start[row + wm + 1u], n);
-    for (uint32_t e = e0; e < e1; ++e) f(e);
-    e0 = w.cell_start[row], e1 = min(w.cell_start[row + x2 + 1u], n);
-    for (uint32_t e = e0; e < e1; ++e) f(e);
+    if (x0 < x2) {
+      const uint32_t e0 = w.cell_start[row + x0], e1 = min(w.cell_start[row + x2 + 1u], n);
+      for (uint32_t e = e0; e < e1; ++e) f(e);
+    } else {
+      uint32_t e0 = w.cell_start[row + x0], e1 = min(w.cell_start[row + wm + 1u], n);
+      for (uint32_t e = e0; e < e1; ++e) f(e);
+      e0 = w.cell_start[row], e1 = min(w.cell_start[row + x2 + 1u], n);
+      for (uint32_t e = e0; e < e1; ++e) f(e);
+    }
   }
 }
 
@@ -715,7 +724,7 @@ __global__ void __launch_bounds__(GEN_THREADS) k_collider_contacts(WorldDev w, c
     Contact* out = w.clist + (size_t)c * CL_CAP;
     uint32_t n = 0;
     bool slow = false;
-    for_each_candidate(w, wp, s, [&](uint32_t q) {
+    for_each_candidate<true>(w, wp, s, [&](uint32_t q) {
       const float4 o = w.sorted[q];
       const uint32_t c2 = __float_as_uint(o.w);
       if (c2 == c || c2 >= w.n_cols) return;
