@@ -712,11 +712,11 @@ __global__ void __launch_bounds__(GEN_THREADS) k_collider_contacts(WorldDev w, c
   uint32_t ncontacts = 0, npush = 0;
   if (e < w.n_cols) {
     const float4 me = w.sorted[e];
-    uint32_t b = w.sorted_parent[e], c = __float_as_uint(me.w);
-    if (c >= w.n_cols || b >= w.n_bodies) {  // a slot that the scatter did not write
+    const uint32_t b = w.sorted_parent[e];  // (of a slot that no scatter wrote: 0)
+    uint32_t c = __float_as_uint(me.w);
+    if (c >= w.n_cols) {
       set_status(w, ST_BAD_INDEX);
       c = 0;
-      b = w.col_parent[0];
     }
     const WorldParam wp = load_wparam(w, MW ? w.col_world[c] : 0u);
     const float2 s = v2(me.x, me.y);  // the snapshot and radius of collider c
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(GEN_THREADS) k_collider_contacts(WorldDev w, c
       // squared-distance pre-test; the exact test is made in contact_pair
       if (!near_pair(s.x - s2.x, s.y - s2.y, r + o.z)) return;
       const uint32_t b2 = w.sorted_parent[q];
-      if (b2 == b || b2 >= w.n_bodies) return;
+      if (b2 == b) return;
       if (!((w.col_memb[c] & w.col_filt[c2]) != 0u && (w.col_memb[c2] & w.col_filt[c]) != 0u)) return;
       const bool sens_any = (w.col_sensor[c] != 0) || (w.col_sensor[c2] != 0);
       PairOut po;

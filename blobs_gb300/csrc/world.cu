@@ -1920,6 +1920,8 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_count, 0, sizeof(uint32_t) * (size_t)h.n_cells, s);
   if (e == cudaSuccess && !res.empty()) e = cudaMemsetAsync(d.cell_count_b, 0, 2 * sizeof(uint32_t) * (size_t)h.n_cells, s);
   if (e == cudaSuccess && !sorted_storage) e = cudaMemsetAsync(d.bslow, 0, nb, s);
+  // a slot that the scatter refuses then still holds a body's index
+  if (e == cudaSuccess && !sorted_storage) e = cudaMemsetAsync(d.sorted_parent, 0, sizeof(uint32_t) * (size_t)nc, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(Counters), s);
   if (e == cudaSuccess && sorted_storage) e = cudaMemsetAsync(d.defer_count, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) {
