@@ -1113,6 +1113,93 @@ __global__ void __launch_bounds__(JB_THREADS) k_joint_blocks(WorldDev w, float2*
   }
 }
 
+// The same three passes through a component's solves one after the other, a
+// thread to a component, up to JB_ITERS iterations: where levels save too
+// little (joint_levels).  Solve (joint q, iteration it) is at it * njoint + q.
+// (A kernel of its own: in one with the levels it cost them 1 us a launch.)
+__global__ void __launch_bounds__(JB_THREADS) k_joint_turns(WorldDev w, float2* __restrict__ pos, float dt,
+                                                            uint32_t iterations) {
+  __shared__ float2 s_pos[JB_BODIES];
+  __shared__ float s_rot[JB_BODIES];
+  __shared__ float4 s_anc[JB_JOINTS];
+  __shared__ float4 s_coef[JB_JOINTS];
+  __shared__ uint32_t s_loc[JB_JOINTS];
+  __shared__ float2 s_dp[JB_ITERS * JB_JOINTS];  // per solve: dp, then rc in .x
+  __shared__ uint8_t s_on[JB_ITERS * JB_JOINTS];  // the solve was applied (not skipped)
+  const uint32_t k = blockIdx.x;
+  const uint32_t b0 = w.jb_body_start[k], nbody = min(w.jb_body_start[k + 1] - b0, JB_BODIES);
+  const uint32_t c = w.jb_comp_start[k] + threadIdx.x, c1 = w.jb_comp_start[k + 1];
+  const uint32_t qa = w.jb_joint_start[c - threadIdx.x], njoint = min(w.jb_joint_start[c1] - qa, JB_JOINTS);
+  const uint32_t nop = min(iterations, JB_ITERS) * njoint;
+#pragma unroll
+  for (uint32_t r = 0; r < (JB_BODIES + JB_THREADS - 1) / JB_THREADS; ++r) {
+    const uint32_t i = threadIdx.x + r * JB_THREADS;
+    if (i < nbody) {
+      const uint32_t body = w.jb_bodies[b0 + i];
+      s_pos[i] = pos[body];
+      s_rot[i] = w.rot[body];
+    }
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < (JB_JOINTS + JB_THREADS - 1) / JB_THREADS; ++r) {
+    const uint32_t i = threadIdx.x + r * JB_THREADS;
+    if (i < njoint) {
+      s_anc[i] = w.jnt_anc[qa + i];
+      s_coef[i] = w.jnt_coef[qa + i];
+      s_loc[i] = w.jnt_local[qa + i];
+    }
+  }
+  for (uint32_t i = threadIdx.x; i < nop; i += JB_THREADS) s_on[i] = 0;
+  __syncthreads();
+  uint32_t q0 = 0, q1 = 0;  // the joints of this thread's component
+  bool bad = false, nan = false;
+  if (c < c1) {
+    q0 = w.jb_joint_start[c] - qa;
+    q1 = w.jb_joint_start[c + 1] - qa;
+    bad = q1 > njoint;
+    for (uint32_t q = q0; q < q1 && !bad; ++q)
+      bad = (s_loc[q] & 0x7fffu) >= nbody || ((s_loc[q] >> 16) & 0x7fffu) >= nbody;
+    if (bad) q1 = q0;
+  }
+  for (uint32_t e0 = 0; e0 < nop; e0 += njoint)
+    for (uint32_t q = q0; q < q1; ++q) {
+      const uint32_t loc = s_loc[q], la = loc & 0x7fffu, lb = (loc >> 16) & 0x7fffu;
+      float2 pa = s_pos[la], pb = s_pos[lb], dp;
+      if (!joint_position(s_anc[q], s_coef[q], loc, pa, pb, dp)) continue;
+      s_pos[la] = pa;
+      s_pos[lb] = pb;
+      s_dp[e0 + q] = dp;
+      s_on[e0 + q] = 1;
+    }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nop; i += JB_THREADS)
+    if (s_on[i]) s_dp[i].x = joint_rotation(s_dp[i], s_coef[i % njoint].w);
+  __syncthreads();
+  for (uint32_t e0 = 0; e0 < nop; e0 += njoint)
+    for (uint32_t q = q0; q < q1; ++q) {
+      if (!s_on[e0 + q]) continue;
+      const uint32_t loc = s_loc[q], la = loc & 0x7fffu, lb = (loc >> 16) & 0x7fffu;
+      const float rc = s_dp[e0 + q].x;
+      const float ra = s_rot[la] + rc * dt;
+      const float rb = s_rot[lb] - rc * dt;
+      s_rot[la] = ra;
+      s_rot[lb] = rb;
+      nan = nan || !isfinite(ra) || !isfinite(rb);
+    }
+  if (bad) set_status(w, ST_BAD_INDEX);
+  if (nan) set_status(w, ST_NAN);
+  __syncthreads();
+#pragma unroll
+  for (uint32_t r = 0; r < (JB_BODIES + JB_THREADS - 1) / JB_THREADS; ++r) {
+    const uint32_t i = threadIdx.x + r * JB_THREADS;
+    if (i < nbody) {
+      const uint32_t body = w.jb_bodies[b0 + i];
+      pos[body] = s_pos[i];
+      w.rot[body] = s_rot[i];
+    }
+  }
+}
+
 template <bool MW, bool SPR, bool PEND, bool SINGLE>
 __global__ void __launch_bounds__(GEN_THREADS) k_integrate(WorldDev w, const float2* __restrict__ pos_in,
                                                    float2* __restrict__ pos_out, SubstepArgs args) {
@@ -1247,9 +1334,10 @@ uint32_t launch_contacts(const WorldDev& w, const float2* pos_in, float2* pos_ou
   return 1u;
 }
 
-void launch_joint_blocks(const WorldDev& w, float2* pos, float dt, uint32_t iterations, cudaStream_t st) {
+void launch_joint_blocks(const WorldDev& w, float2* pos, float dt, uint32_t iterations, bool levels, cudaStream_t st) {
   if (!w.n_jblocks) return;
-  k_joint_blocks<<<w.n_jblocks, JB_THREADS, 0, st>>>(w, pos, dt, iterations);
+  if (levels || iterations > JB_ITERS) k_joint_blocks<<<w.n_jblocks, JB_THREADS, 0, st>>>(w, pos, dt, iterations);
+  else k_joint_turns<<<w.n_jblocks, JB_THREADS, 0, st>>>(w, pos, dt, iterations);
 }
 
 void launch_joints(const WorldDev& w, float2* pos, uint32_t j0, uint32_t j1, float dt, cudaStream_t st) {

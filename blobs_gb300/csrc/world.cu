@@ -225,6 +225,7 @@ struct blobs_world {
   bool keys_valid = false;     // the keys, ranks and cell counts are those of the current snapshots
   bool cells_counted = false;  // cell_count holds counts, whether or not they are those
   bool mass4r = false;          // sorted storage, every body's mass = 4 x radius
+  bool jb_use_levels[JB_ITERS] = {};  // joint blocks run by levels with 1, 2, .. iterations
   std::vector<uint32_t> colour_offsets;  // colour k = joints [colour_offsets[k], colour_offsets[k+1]) in processing order
   std::vector<uint32_t> joint_order;     // processing position -> arena index
   float old_dt = 1.0f;
@@ -402,6 +403,7 @@ struct HostScene {
   std::vector<uint32_t> colour_offsets, joint_order;
   std::vector<uint32_t> jb_comp_start, jb_joint_start, jb_body_start, jb_bodies, jnt_local, jb_level_start;
   std::vector<uint16_t> jb_op, jb_level;
+  bool jb_use_levels[JB_ITERS] = {};
   uint32_t n_cells = 0;
   bool single = false, rot_dynamic = false, pending = false, any_dynamic = false;
 };
@@ -439,10 +441,22 @@ bool check_offsets(const uint32_t* off, uint32_t nw, uint32_t total) {
 // last level that touched one of its two bodies, so running the levels in
 // turn, each in any order, gives every body its solves in the sweep's order;
 // the solves of the first I iterations alone keep that order too.
+//
+// use_levels[I - 1]: whether I iterations run by levels, or a thread to a
+// component that solves one after the other.  A level with its barrier takes
+// about 1.5 times as long as a solve in turn, so a block's levels have to be
+// two thirds of its longest component's solves at most; blocks that are all on
+// the GPU at once (four to an SM) take as long as the slowest, more of them as
+// long as their sum.  50k bodies in chains of 60 joints, us a step by levels /
+// in turn: four iterations (66 levels for 240 solves) 695 / 1325, two 695 /
+// 815, one 680 / 533; in stars of 60 (no two solves together) 1340 / 949,
+// 1098 / 669, 2075 / 1583.  Decided block by block, the two kinds were two
+// launches in a row or one kernel that cost the levels 1 us a launch.
 struct JointSchedule {
   std::vector<uint32_t> joint_order, colour_offsets, jb_comp_start, jb_joint_start, jb_body_start, jb_bodies,
       jnt_local, jb_level_start;
   std::vector<uint16_t> jb_op, jb_level;
+  bool use_levels[JB_ITERS] = {};
 };
 
 void joint_levels(JointSchedule& js) {
@@ -450,13 +464,17 @@ void joint_levels(JointSchedule& js) {
   js.jb_level_start.assign(1, 0u);
   js.jb_level.clear();
   js.jb_op.clear();
+  const bool one_wave = n_blocks <= 4 * 152;
+  uint64_t cost[JB_ITERS][2] = {};  // by levels, in turn
   std::vector<uint32_t> last, level, first;
   for (size_t k = 0; k < n_blocks; ++k) {
     const uint32_t q0 = js.jb_joint_start[js.jb_comp_start[k]], q1 = js.jb_joint_start[js.jb_comp_start[k + 1]];
     last.assign(js.jb_body_start[k + 1] - js.jb_body_start[k], 0u);
     level.clear();
-    uint32_t n_levels = 0;
-    for (uint32_t it = 0; it < JB_ITERS; ++it)
+    uint32_t n_levels = 0, longest = 0;
+    for (uint32_t c = js.jb_comp_start[k]; c < js.jb_comp_start[k + 1]; ++c)
+      longest = std::max(longest, js.jb_joint_start[c + 1] - js.jb_joint_start[c]);
+    for (uint32_t it = 0; it < JB_ITERS; ++it) {
       for (uint32_t q = q0; q < q1; ++q) {
         const uint32_t a = js.jnt_local[q] & 0xffffu, b = js.jnt_local[q] >> 16;
         const uint32_t l = std::max(last[a], last[b]);
@@ -464,6 +482,10 @@ void joint_levels(JointSchedule& js) {
         level.push_back(l);
         n_levels = std::max(n_levels, l + 1);
       }
+      const uint64_t by_levels = 3ull * n_levels, in_turn = 2ull * (it + 1) * longest;
+      cost[it][0] = one_wave ? std::max(cost[it][0], by_levels) : cost[it][0] + by_levels;
+      cost[it][1] = one_wave ? std::max(cost[it][1], in_turn) : cost[it][1] + in_turn;
+    }
     first.assign(n_levels + 1, 0u);
     for (uint32_t l : level) first[l + 1]++;
     for (uint32_t l = 0; l < n_levels; ++l) first[l + 1] += first[l];
@@ -474,6 +496,7 @@ void joint_levels(JointSchedule& js) {
     for (uint32_t i = 0; i < (uint32_t)level.size(); ++i)
       js.jb_op[base + first[level[i]]++] = (uint16_t)((i % (q1 - q0)) | ((i / (q1 - q0)) << JB_OP_BITS));
   }
+  for (uint32_t it = 0; it < JB_ITERS; ++it) js.use_levels[it] = cost[it][0] <= cost[it][1];
 }
 
 // The joint processing schedule (see JointSchedule).  The bodies a chain
@@ -807,6 +830,7 @@ int build_host_scene(const blobs_config& cfg, float cell_scale, const blobs_scen
     h.jb_op = std::move(js.jb_op);
     h.jb_level = std::move(js.jb_level);
     h.jb_level_start = std::move(js.jb_level_start);
+    std::copy(js.use_levels, js.use_levels + JB_ITERS, h.jb_use_levels);
   }
   h.jnt_a.resize(nj);
   h.jnt_b.resize(nj);
@@ -1191,7 +1215,8 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
   auto joints = [&](float2* p) {
     mark_begin(w, PHASE_JOINTS);
     if (d.n_jblocks && w->cfg.joint_iterations) {
-      launch_joint_blocks(d, p, dt, w->cfg.joint_iterations, st);
+      const uint32_t it = w->cfg.joint_iterations;
+      launch_joint_blocks(d, p, dt, it, it <= JB_ITERS && w->jb_use_levels[it - 1], st);
       w->enqueued += 1;
     }
     for (uint32_t it = 0; it < w->cfg.joint_iterations; ++it)
@@ -1968,6 +1993,7 @@ int blobs_world_load(blobs_world* w, const blobs_scene* scene, float old_dt) {
   w->keys_valid = w->cells_counted = false;
   w->colour_offsets = h.colour_offsets;
   w->joint_order = h.joint_order;
+  std::copy(h.jb_use_levels, h.jb_use_levels + JB_ITERS, w->jb_use_levels);
   w->old_dt = old_dt;
   w->time = 0.0;
   w->accumulator = 0.0;
