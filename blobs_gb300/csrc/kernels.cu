@@ -451,7 +451,7 @@ __device__ __forceinline__ void integrate_body(const WorldDev& w, uint32_t b, fl
 // longest rows (k_collider_contacts, 200k bodies, four steps: 3.24 -> 3.17 ms;
 // records loaded two or four at a time were slower, 3.31 and 3.27).  The walks
 // over crowded bodies are long rows, and pay for the choice of row at each
-// candidate (50k bodies at 16 times that density: 11.9 ms a step by rows,
+// candidate (50k bodies at 16 times that density: 11.6 ms a step by rows,
 // 12.7 flat).
 template <bool FLAT = false, class F>
 __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const WorldParam& wp, float2 s, F&& f) {
@@ -475,18 +475,15 @@ __device__ __forceinline__ void for_each_candidate(const WorldDev& w, const Worl
     for (uint32_t t = 0; t < m; ++t) f(t < l0 ? b[0] + t : (t < l0 + l1 ? b[1] + (t - l0) : b[2] + (t - l0 - l1)));
     return;
   }
+  // row by row, a wrapping one in two ranges
 #pragma unroll 1
-  for (int oy = -1; oy <= 1; ++oy) {
-    const uint32_t row = wp.cell_base + (((iy + (uint32_t)oy) & hm) << wp.log2w);
-    if (x0 < x2) {
-      const uint32_t e0 = w.cell_start[row + x0], e1 = min(w.cell_start[row + x2 + 1u], n);
-      for (uint32_t e = e0; e < e1; ++e) f(e);
-    } else {
-      uint32_t e0 = w.cell_start[row + x0], e1 = min(w.cell_start[row + wm + 1u], n);
-      for (uint32_t e = e0; e < e1; ++e) f(e);
-      e0 = w.cell_start[row], e1 = min(w.cell_start[row + x2 + 1u], n);
-      for (uint32_t e = e0; e < e1; ++e) f(e);
-    }
+  for (uint32_t k = 0; k < 6u; ++k) {
+    const uint32_t row = wp.cell_base + (((iy + (k >> 1) - 1u) & hm) << wp.log2w);
+    const bool second = k & 1u, wraps = x0 >= x2;
+    if (second && !wraps) continue;
+    const uint32_t e0 = w.cell_start[row + (second ? 0u : x0)];
+    const uint32_t e1 = min(w.cell_start[row + (second || !wraps ? x2 : wm) + 1u], n);
+    for (uint32_t e = e0; e < e1; ++e) f(e);
   }
 }
 
