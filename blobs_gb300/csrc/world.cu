@@ -932,6 +932,36 @@ int build_host_scene(const blobs_config& cfg, float cell_scale, const blobs_scen
 constexpr uint32_t RES_BLOCKS = 2 * 152;
 constexpr uint32_t RES_LARGEST[RES_PER_THREAD] = {2048u, 1024u};
 
+// And a world must not crowd: a body with more than 64 candidates in its 3x3
+// cells takes a warp of its own (deferred_body), of which the kernels of a
+// substep have 2,432 and a cluster 8 a block.  Cells are as wide as the
+// largest body, so one large body among small ones is enough.  The candidates
+// to be expected are those of a pile (0.85 of the area covered) of the
+// world's radii, or of a box or circle that is too small for its bodies; a
+// world whose bodies all come together otherwise is not foreseen.  Settled,
+// us a step, kernels / resident, one body of 1.6, 2, 3 and 6 times the largest
+// of the others (53, 83, 186 and 720 candidates in a pile of 2,000): 2,000
+// bodies 229 / 177, 236 / 464, 203 / 798, 153 / 1,298; 1,000 bodies 185 / 123,
+// 215 / 310, 198 / 733, 150 / 1,146; 200 bodies (one block) 117 / 55, 173 /
+// 124, 172 / 442, 125 / 647.  Boxes overfilled 2, 3 and 4 times (49, 73, 98
+// candidates): 2,000 bodies 357 / 305, 445 / 656, 476 / 1,006; 500 bodies
+// 243 / 189, 336 / 300, 378 / 588; 200 bodies 205 / 148, 255 / 200, 321 / 291.
+constexpr double RES_CROWD_PILE = 64.0, RES_CROWD_BOX = 80.0, RES_CROWD_BLOCK = 96.0;
+
+bool crowds(const HostScene& h, const blobs_scene& s, uint32_t world, uint32_t b0, uint32_t b1) {
+  const WorldParam& wp = h.wparam[world];
+  const double pi = 3.14159265358979, n = b1 - b0, block = 9.0 * (double)wp.cs * wp.cs;
+  double covered = 0.0, box = INFINITY;
+  for (uint32_t i = b0; i < b1; ++i) covered += pi * (double)h.col_radius[i] * h.col_radius[i];
+  if (wp.has_box) box = ((double)wp.box_hi_x - wp.box_lo_x) * ((double)wp.box_hi_y - wp.box_lo_y);
+  for (uint32_t k = 0; k < s.n_circles; ++k) box = std::min(box, pi * (double)s.circles[3 * k + 2] * s.circles[3 * k + 2]);
+  const bool one_block = b1 - b0 <= RES_THREADS;
+  auto too_many = [&](double candidates, double most) {  // (no area: NaN or infinite)
+    return !(candidates <= (one_block ? RES_CROWD_BLOCK : most)) && !(n <= (one_block ? RES_CROWD_BLOCK : most));
+  };
+  return too_many(block * 0.85 * n / covered, RES_CROWD_PILE) || too_many(block * n / box, RES_CROWD_BOX);
+}
+
 void resident_classes(const HostScene& h, const blobs_scene& s, uint32_t nw, std::vector<ResWorld>& worlds,
                       std::vector<blobs_world::ResClass>& classes) {
   auto body0 = [&](uint32_t k) { return nw > 1 ? s.world_body_offsets[k] : (k ? s.n_bodies : 0u); };
@@ -940,6 +970,7 @@ void resident_classes(const HostScene& h, const blobs_scene& s, uint32_t nw, std
     largest = std::max(largest, body0(k + 1) - body0(k));
     if (h.wparam[k].log2w + h.wparam[k].log2h > 30u) return;
     if ((1u << (h.wparam[k].log2w + h.wparam[k].log2h)) > RES_MAX_CELLS) return;
+    if (crowds(h, s, k, body0(k), body0(k + 1))) return;
   }
   auto blocks = [](uint32_t n, uint32_t per) {
     uint32_t c = 1;
