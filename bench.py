@@ -343,9 +343,20 @@ def run_reference(args):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
+def load_captured(w, scene, dt):
+    """The scene's initial state in a world whose step graphs exist: a step is
+    launched kernel by kernel the first time from a storage buffer, captured
+    the second and replayed after that."""
+    w.load(scene)
+    w.snapshot()
+    for _ in range(5):  # the first step, then both buffers twice
+        w.step(dt)
+    w.restore()
+
+
 def batched_comparison(dev, steps=100, sample=1024, seed=4):
-    """4,096 uneven worlds stepped as one batch (a 100-step rollout captured
-    in one CUDA graph) against the per-world form (each world its own device
+    """4,096 uneven worlds stepped as one batch (a 100-step rollout replayed
+    as one CUDA graph) against the per-world form (each world its own device
     world and its own 100-step rollout launch), timed on `sample` evenly
     spaced worlds -- each created, captured, timed and closed in turn -- and
     scaled to all 4,096 by body count."""
@@ -361,7 +372,8 @@ def batched_comparison(dev, steps=100, sample=1024, seed=4):
     cell_scale = w.autotune(scene, dt, trial_steps=3)
     for _ in range(3):
         w.step(dt)
-    w.rollout(dt, steps)  # capture
+    for _ in range(2):
+        w.rollout(dt, steps)  # launched, captured
     torch.cuda.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record(stream)
@@ -379,7 +391,8 @@ def batched_comparison(dev, steps=100, sample=1024, seed=4):
         ww.set_stream(stream.cuda_stream)
         for _ in range(3):
             ww.step(dt)
-        ww.rollout(dt, steps)  # capture
+        for _ in range(2):
+            ww.rollout(dt, steps)  # launched, captured
         torch.cuda.synchronize()
         e0.record(stream)
         ww.rollout(dt, steps)
@@ -487,7 +500,7 @@ def sparse_comparison(dev, seed=1):
     stream = torch.cuda.current_stream(dev)
     w = native.World(scene, device=dev.index)
     w.set_stream(stream.cuda_stream)
-    w.rollout(scene.dt, scene.n_steps)  # capture the graphs
+    w.rollout(scene.dt, scene.n_steps)  # warm-up
     w.load(scene)
     torch.cuda.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -515,7 +528,7 @@ def sparse_comparison(dev, seed=1):
 def events_comparison(dev, settle=200, steps=5, seed=2):
     """The headline world with the CollisionEvent stream on (physics.rs:304-311:
     one event per contact per substep): `settle` steps from t = 0 without
-    events, one untimed step with them (the step graphs are captured again),
+    events, four untimed steps with them (the step graphs are captured again),
     then `steps` steps with them -- each step between its own
     CUDA-event pair (L2 flushed before it), its events drained to the host
     and put in the reference's order after it (host time, outside the
@@ -529,16 +542,17 @@ def events_comparison(dev, settle=200, steps=5, seed=2):
     w.set_stream(stream.cuda_stream)
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.float32, device=dev)
     out = {}
+    lead = 4
     for on in (False, True):
         w.load(scene)
         for _ in range(settle):
             w.step(scene.dt)
         if on:
             w.set_events(True, capacity=12_000_000)
-            w.step(scene.dt)  # the step graphs are captured again with the stream on (untimed)
-            w.drain_events()
-        else:
+        for _ in range(lead):  # the step graphs are captured again with the stream on (untimed)
             w.step(scene.dt)
+            if on:
+                w.drain_events()
         ms, drain_s, n_events = [], [], 0
         for _ in range(steps):
             flush.zero_()
@@ -559,10 +573,10 @@ def events_comparison(dev, settle=200, steps=5, seed=2):
         else:
             out["events_off"] = {"ms_per_step": float(np.mean(ms))}
     w.close()
-    out.update({"bodies": scene.n_bodies, "steps": "%d-%d of the rollout" % (settle + 1, settle + steps),
+    out.update({"bodies": scene.n_bodies, "steps": "%d-%d of the rollout" % (settle + lead + 1, settle + lead + steps),
                 "note": "device time per step with the stream on (the contact kernels append one 32-byte record "
-                        "per contact) and off; the drain copies the step's events to the host and sorts them "
-                        "into the reference's order"})
+                        "per contact) and off; the drain puts the step's events into the reference's order on "
+                        "the device and copies them to the host"})
     return out
 
 
@@ -571,8 +585,8 @@ def adjoint_comparison(dev, steps=120, every=16, seed=5, finite_steps=32):
     pass (one CUDA-graph rollout) against the same rollout recorded with a
     checkpoint every 16 steps plus the backward pass (recompute each
     segment, then the adjoint substeps in reverse).  Every timed leg starts
-    from the scene's initial state (the world is reloaded before it) and
-    covers steps 0-119; each leg runs once untimed first (graph capture).
+    from the scene's initial state (restored before it) and covers steps
+    0-119; each leg runs twice untimed first (launches, graph capture).
     The same legs are timed over the first `finite_steps` steps, a horizon
     whose gradients stay finite in f32."""
     import numpy as np
@@ -583,6 +597,7 @@ def adjoint_comparison(dev, steps=120, every=16, seed=5, finite_steps=32):
     stream = torch.cuda.current_stream(dev)
     w = native.World(scene, device=dev.index)
     w.set_stream(stream.cuda_stream)
+    w.snapshot()
     M = sum(len(m) for m in marked)
     idx = np.concatenate([int(scene.world_body_offsets[i]) + m for i, m in enumerate(marked)])
     tgt = np.concatenate(targets).astype(np.float64)
@@ -596,15 +611,15 @@ def adjoint_comparison(dev, steps=120, every=16, seed=5, finite_steps=32):
     def legs(n):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         out = {}
-        for timed in (False, True):
-            w.load(scene)
+        for timed in (False, False, True):
+            w.restore()
             torch.cuda.synchronize()
             e0.record(stream)
             w.rollout(dt, n)
             e1.record(stream)
             torch.cuda.synchronize()
             fwd = e0.elapsed_time(e1)
-            w.load(scene)
+            w.restore()
             torch.cuda.synchronize()
             e0.record(stream)
             w.rollout_record(dt, n, every)
@@ -633,7 +648,7 @@ def adjoint_comparison(dev, steps=120, every=16, seed=5, finite_steps=32):
             "checkpoint_every": every, "fwd_ms": full["fwd_ms"], "fwd_record_ms": full["fwd_record_ms"],
             "bwd_ms": full["bwd_ms"], "fwd_bwd_over_fwd": full["fwd_bwd_over_fwd"],
             "gradients_finite": full["gradients_finite"],
-            "window": "every leg from the scene's initial state (reloaded before it): steps 0-%d" % (steps - 1),
+            "window": "every leg from the scene's initial state (restored before it): steps 0-%d" % (steps - 1),
             "finite_horizon": short, "cpu_baseline": cpu,
             "note": "the derivative of this contact dynamics grows by orders of magnitude every few steps "
                     "(max |dL/dv0| of one world: 4e-2 at step 10, 1e1 at 15, 1e12 at 40, 1e84 at 120, f64), so "
@@ -687,7 +702,7 @@ def run_ours(args):
 
     # -- timed region: the whole rollout from t = 0, every step between its own
     # CUDA-event pair, L2 flushed before each; the K steps at `timed` make `value`
-    world.load(scene)
+    load_captured(world, scene, dt)
     starts = [torch.cuda.Event(enable_timing=True) for _ in range(n_steps)]
     ends = [torch.cuda.Event(enable_timing=True) for _ in range(n_steps)]
     counts = {}
@@ -745,7 +760,7 @@ def run_ours(args):
     h_pos = torch.empty((n, 2), dtype=torch.float32, pin_memory=True).numpy()
     h_old = torch.empty((n, 2), dtype=torch.float32, pin_memory=True).numpy()
     h_vel = torch.empty((n, 2), dtype=torch.float32, pin_memory=True).numpy()
-    world.load(scene)
+    load_captured(world, scene, dt)
     e2e_s = []
     for i in range(n_steps):
         if i not in timed_set:
