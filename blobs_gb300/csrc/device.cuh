@@ -23,7 +23,7 @@ enum : uint8_t {
 // Device status bits, read back by the host after a synchronising call.
 enum : uint32_t {
   ST_NAN = 1u,         // NaN contact normal or non-finite rotation (physics.rs:293, 471-474)
-  ST_TIMEOUT = 2u,     // a bounded spin-wait gave up (reserved: no kernel waits on another)
+  ST_TIMEOUT = 2u,     // a bounded spin-wait gave up (reserved: no kernel spins)
   ST_BAD_INDEX = 4u,   // a device bounds check fired
 };
 
@@ -149,8 +149,8 @@ struct WorldDev {
   uint32_t* defer_count;     // entries of defer_list this substep (zeroed by the cell scan)
 
   // collision event stream (NULL when off): one record per resolved pair,
-  // appended in any order and put in the reference's order on the host by
-  // (substep sequence, a, b)
+  // appended in any order and put in the reference's order, (substep sequence,
+  // a, b), by a drain: on the device (events.cu), few of them on the host
   uint4* ev_rec;             // (sequence, collider a, collider b, 0), a > b
   float4* ev_vel;            // (impact_vel_a, impact_vel_b): calculated_velocity of the parents
   uint32_t* ev_count;        // appended so far (may exceed ev_cap: overflow)
@@ -363,7 +363,7 @@ struct ResidentArgs {
 // a > b in collider order and the parents' calculated_velocity at the start
 // of the contact pass.
 // The lanes of a warp that append together take their slots with one atomic
-// (the buffer is put in order on the host, so any order of slots will do).
+// (the buffer is put in order when it is drained, so any order of slots will do).
 __device__ __forceinline__ void record_event(const WorldDev& w, uint32_t a, uint32_t b, float2 va, float2 vb) {
   const uint32_t active = __activemask();
   const uint32_t lane = threadIdx.x & 31u;
@@ -382,7 +382,7 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr uint32_t SCAN_ONE_THREADS = 1024;  // k_scan_one
-constexpr uint32_t SCAN_ONE_ROWS = 4;
+constexpr uint32_t SCAN_ONE_ROWS = 2;
 constexpr uint32_t SCAN_ONE_CELLS = SCAN_ONE_THREADS * 4 * SCAN_ONE_ROWS;
 constexpr uint32_t SCAN_PREFIX_TILES = 256;  // more tiles: their prefix by one k_tile_prefix block
 constexpr int CONTACT_LIST = 24;           // per-body sorted contact list kept in registers

@@ -17,7 +17,8 @@
 //                      integration when there are no joints
 //   k_contact_single   both passes in one for single-collider bodies
 //   k_joint_blocks     the small joint components, each swept alone in the
-//                      reference's order in shared memory
+//                      reference's order in shared memory, by levels
+//                      (k_joint_turns: a thread to a component)
 //   k_joints           one colour of the large components' joints
 //   k_integrate        Verlet + collider snapshot + constraints, and the cell
 //                      key / rank of every collider for the next substep
@@ -238,9 +239,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(WorldDev w) {
 }
 
 // Few cells: the whole scan by one block, one launch instead of two that are
-// each mostly launch and first loads (a frame of 20,000 spheres, 16,384 cells:
-// 0.48 -> 0.45 ms).  A warp takes up to SCAN_ONE_ROWS consecutive rows of 128
-// cells, all of its loads in flight.
+// each mostly launch and first loads.  A warp takes up to SCAN_ONE_ROWS
+// consecutive rows of 128 cells, all of its loads in flight.  Worlds of 2,500 to
+// 20,000 spheres, us a step with one block up to 4,096 / 8,192 / 16,384 cells:
+// 4,096 cells 88.6 / 88.9 / 88.8, 8,192 cells 140.1 / 130.1 / 131.9, 16,384
+// cells 100.2 / 100.0 / 103.1 (10,000 spheres 215.8 / 215.8 / 218.6, 20,000
+// 264.6 / 264.3 / 266.5).
 __global__ void __launch_bounds__(SCAN_ONE_THREADS) k_scan_one(WorldDev w) {
   pdl_enter();
   __shared__ uint32_t s_warp[SCAN_ONE_THREADS / 32];

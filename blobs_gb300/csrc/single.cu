@@ -948,7 +948,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
     __syncwarp();
     if ((HOOKS & HOOK_EVENTS) && w.ev_rec) {
       // the body's events (its contacts with lower ids), appended by all
-      // lanes; the host puts the buffer in the reference's order
+      // lanes; a drain puts the buffer in the reference's order (events.cu)
       const uint32_t seq = *w.ev_seq;
       const float2 va = a.v_in[j];
       for (uint32_t e0 = 0; e0 < cnt; e0 += 32u) {

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) k_sh_offsets(const uint32_t* start, uint3
 
 inline uint32_t nblk(uint64_t n) { return (uint32_t)((n + 255u) / 256u); }
 
-// The two-kernel cell scan of kernels.cu over an arbitrary count array:
+// The cell scan of kernels.cu over an arbitrary count array:
 // start[k] = sum(count[0..k)), start[n] = total, count zeroed.
 void scan_counts(uint32_t* count, uint32_t* start, uint32_t n, uint32_t* tile_sums, uint32_t* sub_bins,
                  cudaStream_t st) {

@@ -1435,7 +1435,7 @@ uint32_t f2bits(float f) {
 }
 
 // `n_steps` steady-state steps (no pending request, old_dt == step delta)
-// from one cached CUDA graph.
+// from one cached CUDA graph (the first time launched one by one).
 int launch_steady(blobs_world* w, float delta, uint32_t n_steps) {
   const float step_delta = delta / (float)w->cfg.substeps;
   const bool coll = w->cfg.collisions_enabled && w->nc > 0;

@@ -46,7 +46,7 @@ typedef enum blobs_status {
   BLOBS_ERR_OVERFLOW = 3,         /* a caller-provided capacity was too small */
   BLOBS_ERR_NAN = 4,              /* NaN contact normal / non-finite rotation (physics.rs:293,471-474) */
   BLOBS_ERR_CUDA = 5,             /* a CUDA runtime call failed */
-  BLOBS_ERR_TIMEOUT = 6,          /* a bounded device-side wait gave up (reserved: no kernel waits on another) */
+  BLOBS_ERR_TIMEOUT = 6,          /* a bounded device-side wait gave up (reserved: no kernel spins) */
   BLOBS_ERR_NO_DEVICE = 7,        /* no usable CUDA device */
   BLOBS_ERR_OUT_OF_MEMORY = 8,    /* device allocation failed */
   BLOBS_ERR_STATE = 9             /* call not valid in the world's current state */
@@ -297,7 +297,8 @@ int blobs_world_rollout_record(blobs_world* w, double delta, uint32_t n_steps, u
  * in a fixed order: the gradients are deterministic.  Its scratch is 92 B per
  * body per substep of one checkpoint segment (the state after the substep
  * and up to 16 recorded contacts), taken for the call from a pool that keeps
- * up to 8 GB per device for the next one; a body with more than
+ * up to 8 GB per device for the next one, until the device's last world is
+ * destroyed; a body with more than
  * 16 contacts in one substep gives BLOBS_ERR_OVERFLOW.  The derivative of
  * long contact-rich rollouts can exceed the f32 range; such gradients come
  * back as +-inf or NaN with BLOBS_OK.  Synchronising. */
