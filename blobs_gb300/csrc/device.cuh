@@ -323,6 +323,7 @@ struct SingleArgs {
   const float4* cand;        // candidate records in cell order
   const uint32_t* own_cell;  // cell of each storage slot in this substep's order
   const uint32_t* cell_start;  // the substep's cell table (indexed by global cell),
+  uint32_t slot_end;           // whose ranges, whatever the counts are, are taken to end here at the latest,
   uint32_t* cell_count;        // the counts of the next substep,
   uint32_t* key_out;           // the bodies' cells and ranks there,
   uint32_t* rank_out;

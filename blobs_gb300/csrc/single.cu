@@ -692,7 +692,7 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
       // Cells away from the grid edge: the 3x3 block is three contiguous
       // ranges of the cell-order array, one per row.
       const float4* C = a.cand;
-      const uint32_t n = w.n_bodies;
+      const uint32_t n = a.slot_end;
       const uint32_t r1 = own_key - 1u, r0 = r1 - (wm + 1u), r2 = r1 + (wm + 1u);
       const uint32_t s0 = a.cell_start[r0], s1 = a.cell_start[r1], s2 = a.cell_start[r2];
       const uint32_t e0 = min(a.cell_start[r0 + 3u], n), e1 = min(a.cell_start[r1 + 3u], n),
@@ -730,7 +730,7 @@ __device__ __forceinline__ bool step_slot(const WorldDev& w, const SingleArgs& a
     } else if (a.contacts) {
       // cells on the grid edge (the torus wraps): general segments
       const float4* C = a.cand;
-      const Segments g = segments(a.cell_start, w.n_bodies, wp, own_key);
+      const Segments g = segments(a.cell_start, a.slot_end, wp, own_key);
       const uint32_t total = g.l[0] + g.l[1] + g.l[2] + g.l[3] + g.l[4] + g.l[5];
       if (total <= 64u) {
         // Phase 1: one squared-distance test per candidate (self included:
@@ -912,7 +912,7 @@ __device__ __forceinline__ void deferred_body(const WorldDev& w, const SingleArg
   const BodyConst k = body_const<MODE>(w, MODE == 3 ? a.wparam[slot_world<MODE>(w, j)] : wp0, c, r);
   const WorldParam wp = MODE == 2 ? a.wparam[k.world] : (MODE == 3 ? a.wparam[slot_world<MODE>(w, j)] : wp0);
   const float2 p0 = v2(bv.x, bv.y);
-  const Segments g = segments(a.cell_start, w.n_bodies, wp, a.own_cell[j]);
+  const Segments g = segments(a.cell_start, a.slot_end, wp, a.own_cell[j]);
   const uint32_t m = g.l[0] + g.l[1] + g.l[2] + g.l[3] + g.l[4] + g.l[5];
   uint32_t cnt = 0;
   for (uint32_t t0 = 0; t0 < m; t0 += 32u) {
@@ -1068,11 +1068,10 @@ __device__ __forceinline__ void cluster_barrier(uint32_t n_blocks) {
   }
 }
 
-// start[k] = first + sum(count[0..k)) for k in [0, n], n a multiple of 4, at
-// most `limit`: whatever the counts are, no range leaves the world's records;
+// start[k] = first + sum(count[0..k)) for k in [0, n], n a multiple of 4;
 // every thread of the block calls it
-__device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, uint32_t first, uint32_t limit,
-                                           uint32_t* start, uint32_t* s_warp) {
+__device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, uint32_t first, uint32_t* start,
+                                           uint32_t* s_warp) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // each warp takes consecutive rows of 128 cells, four to a lane; the first
   // two rows stay in registers (all of them up to 2,048 cells)
@@ -1105,12 +1104,10 @@ __device__ __forceinline__ void block_scan(const uint32_t* count, uint32_t n, ui
       if (lane >= (uint32_t)o) x += y;
     }
     const uint32_t k = r * 128u + lane * 4u, b = run + x - own;
-    if (k < n)
-      *reinterpret_cast<uint4*>(start + k) = make_uint4(min(b, limit), min(b + t.x, limit), min(b + t.x + t.y, limit),
-                                                        min(b + t.x + t.y + t.z, limit));
+    if (k < n) *reinterpret_cast<uint4*>(start + k) = make_uint4(b, b + t.x, b + t.x + t.y, b + t.x + t.y + t.z);
     run += __shfl_sync(0xffffffffu, x, 31);
   }
-  if (warp == RES_WARPS - 1u && lane == 0) start[n] = min(run, limit);
+  if (warp == RES_WARPS - 1u && lane == 0) start[n] = run;
   __syncthreads();
 }
 
@@ -1142,6 +1139,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentAr
     a.cell_start = s_start - wp.cell_base;
     a.wparam = &wp;
     a.cand = s_cand - b0;
+    a.slot_end = b0 + n;
   }
   __syncthreads();
   const uint32_t cell_base = wp.cell_base, n_cells = 1u << (wp.log2w + wp.log2h);
@@ -1195,7 +1193,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(WorldDev w, ResidentAr
       rq[u] = k < n ? rnk[b0 + k] : 0u;
       aq[u] = k < n ? a_cur[b0 + k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    block_scan(count + cell_base, n_cells, b0, b0 + n, s_start, s_warp);
+    block_scan(count + cell_base, n_cells, b0, s_start, s_warp);
     for (;;) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {

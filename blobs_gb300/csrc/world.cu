@@ -1262,6 +1262,7 @@ void enqueue_substep(blobs_world* w, float dt, float old_dt, bool pending, bool 
     SingleArgs a;
     std::memset(&a, 0, sizeof(a));
     a.cell_start = d.cell_start;
+    a.slot_end = w->nb;
     a.cell_count = d.cell_count;
     a.key_out = d.key;
     a.rank_out = d.rank;
