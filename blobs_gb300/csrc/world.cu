@@ -105,12 +105,14 @@ namespace {
 // reverse pass (checkpoints, recorded contacts: 6 GB for 256 x 2,048 bodies
 // and 128 substeps).  One pool per device, shared by every world, stream and
 // thread of the process; freed memory stays in it, up to POOL_KEEP bytes, for
-// the next call, and goes back to the device when an allocation of this
-// library fails and with the device's last world.  (A call that needs more
-// maps the rest and unmaps it again.)  Mapping that memory, clearing it and unmapping it on each
-// call was 5.5 of the 26.9 ms of a recorded forward and backward of the
-// batch above (0.18 of 1.27 ms with 16 x 512 bodies and 8 substeps).
+// the next call (one that needs more maps the rest and unmaps it again), and
+// goes back to the device when an allocation of this library fails and, but
+// for POOL_IDLE, with the device's last world.  Mapping that memory, clearing
+// it and unmapping it on each call was 5.5 of the 26.9 ms of a recorded forward
+// and backward of the batch above (0.18 of 1.27 ms with 16 x 512 bodies and 8
+// substeps).
 constexpr uint64_t POOL_KEEP = 8ull << 30;
+constexpr uint64_t POOL_IDLE = 64ull << 20;
 constexpr int POOL_DEVICES = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[POOL_DEVICES] = {};
@@ -151,7 +153,7 @@ void count_world(int device, bool came) {
   if (device < 0 || device >= POOL_DEVICES) return;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   if (came) ++g_worlds[device];
-  else if (--g_worlds[device] == 0 && g_pools[device]) cudaMemPoolTrimTo(g_pools[device], 0);
+  else if (--g_worlds[device] == 0 && g_pools[device]) cudaMemPoolTrimTo(g_pools[device], POOL_IDLE);
 }
 
 template <class T> cudaError_t pool_alloc(int device, T** p, size_t bytes, cudaStream_t st) {
