@@ -323,7 +323,6 @@ struct SingleArgs {
   const float4* cand;        // candidate records in cell order
   const uint32_t* own_cell;  // cell of each storage slot in this substep's order
   const uint32_t* cell_start;  // the substep's cell table (indexed by global cell),
-  uint32_t slot_end;           // whose ranges, whatever the counts are, are taken to end here at the latest,
   uint32_t* cell_count;        // the counts of the next substep,
   uint32_t* key_out;           // the bodies' cells and ranks there,
   uint32_t* rank_out;
@@ -332,6 +331,7 @@ struct SingleArgs {
   uint32_t contacts, pending, springs, rot_dynamic, do_keys, write_v, move_v;
   uint32_t v_vel;            // V holds calculated_velocity (else the displacement of the last substep)
   uint32_t mass4r;           // every body's mass is 4 x its radius: a partner's mass follows from its candidate record
+  uint32_t slot_end;         // cell ranges, whatever the counts are, are taken to end here at the latest
   // contact recording for the adjoint (NULL in ordinary steps): every
   // contact of body c in the order it was applied (ascending partner id),
   // rec_list[k * n_bodies + c] = partner | pushed << 31 for k < REC_CAP,
